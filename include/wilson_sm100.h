@@ -264,6 +264,11 @@ wl_status wl_random_algebra(wl_ctx* ctx, uint64_t seed, uint64_t stream, int bat
    `accumulate` is non-zero, F += coef * force, else F = coef * force. */
 wl_status wl_pf_force(wl_ctx* ctx, wl_gauge* gauge, const void* X, const void* Y, double coef,
                       int accumulate, void* F);
+/* F = coef * (f(K_oe X_e, Y_e) + f(X_e, K^dag_oe Y_e)) with f the force above: the
+   even-odd force (su3_wilson_nf2.py:1578-1597) for coef = -1/m0^2.  `scratch` holds
+   two fields (2 * volume * 12 complex128), overwritten. */
+wl_status wl_pf_force_eo(wl_ctx* ctx, wl_gauge* gauge, const void* X, const void* Y, double coef,
+                         void* scratch, void* F);
 
 /* Gauge sector (HMC pure-gauge pieces) ------------------------------------ */
 /* Links / momenta in the reference layout BMXYIJ: complex128

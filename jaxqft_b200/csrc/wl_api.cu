@@ -975,25 +975,50 @@ extern "C" wl_status wl_random_algebra(wl_ctx* ctx, uint64_t seed, uint64_t stre
 }
 
 // ============================================================== force
+static wl_status launch_pf_force(wl_ctx* ctx, wl_gauge* G, const void* const (&X)[2], const void* const (&Y)[2],
+                                 double coef, int accumulate, void* F) {
+  const Geom& g = ctx->g;
+  ForceArgs A;
+  A.g = g;
+  A.U = G->d18;
+  uintptr_t any = 0;
+  for (int p = 0; p < 2; ++p) {
+    A.X[p] = (const double*)X[p];
+    A.Y[p] = (const double*)Y[p];
+    any |= (uintptr_t)X[p] | (uintptr_t)Y[p];
+  }
+  A.F = (double2*)F;
+  A.coef = coef;
+  A.accumulate = accumulate;
+  const unsigned blocks = 4u * (unsigned)((g.V + kForceSites - 1) / kForceSites);
+  g_launches++;
+  // sector loads need 32-byte aligned fields (sites are 192 bytes apart)
+  if ((any & 31) == 0) pf_force_kernel<4, true><<<blocks, 2 * kForceSites, 0, ctx->stream>>>(A);
+  else pf_force_kernel<2, false><<<blocks, 2 * kForceSites, 0, ctx->stream>>>(A);
+  return check_launch(ctx, "pf_force_kernel");
+}
+
 extern "C" wl_status wl_pf_force(wl_ctx* ctx, wl_gauge* G, const void* X, const void* Y, double coef, int accumulate,
                                  void* F) {
   NvtxRange nvtx_range("wl_pf_force");
   if (!ctx || !G || !X || !Y || !F) WL_FAIL(ctx, WL_ERR_ARG, "null argument");
   WL_CUDA(ctx, cudaSetDevice(ctx->device));
-  const Geom& g = ctx->g;
-  ForceArgs A;
-  A.g = g;
-  A.U.ptr = G->ref_copy;
-  A.U.V = g.V;
-  A.X = sref(X, g);
-  A.Y = sref(Y, g);
-  A.F = (double2*)F;
-  A.coef = coef;
-  A.accumulate = accumulate;
-  dim3 grid((g.Vh + 127) / 128, 2, 4);
-  g_launches++;
-  pf_force_kernel<<<grid, 128, 0, ctx->stream>>>(A);
-  return check_launch(ctx, "pf_force_kernel");
+  return launch_pf_force(ctx, G, {X, X}, {Y, Y}, coef, accumulate, F);
+}
+
+// coef (f(K_oe X_e, Y_e) + f(X_e, K^dag_oe Y_e)): the two hops into the caller's scratch (two fields; only their
+// odd sites are written), then one force over the fields that are X_e, Y_e on even sites and the hops on odd
+// ones (wl_force.cuh).
+extern "C" wl_status wl_pf_force_eo(wl_ctx* ctx, wl_gauge* G, const void* X, const void* Y, double coef,
+                                    void* scratch, void* F) {
+  NvtxRange nvtx_range("wl_pf_force_eo");
+  if (!ctx || !G || !X || !Y || !scratch || !F) WL_FAIL(ctx, WL_ERR_ARG, "null argument");
+  WL_CUDA(ctx, cudaSetDevice(ctx->device));
+  void* kx = scratch;
+  void* ky = (char*)scratch + (size_t)ctx->g.V * 12 * sizeof(double2);
+  ref_hop<false>(ctx, G, X, kx, nullptr, 0.0, -0.5, 1, 1, 1);
+  ref_hop<true>(ctx, G, Y, ky, nullptr, 0.0, -0.5, 1, 1, 1);
+  return launch_pf_force(ctx, G, {X, kx}, {Y, ky}, coef, 0, F);
 }
 
 // ============================================================== gauge sector

@@ -39,7 +39,7 @@ EXPORTS = (
     "wl_version", "wl_ctx_create", "wl_ctx_destroy", "wl_last_error", "wl_ctx_set_stream",
     "wl_ctx_synchronize", "wl_eo_maps", "wl_gauge_create", "wl_gauge_update", "wl_gauge_unitarity",
     "wl_gauge_destroy", "wl_apply", "wl_solve", "wl_engine_create", "wl_engine_destroy", "wl_engine_admit",
-    "wl_engine_step", "wl_engine_run", "wl_engine_poll", "wl_engine_poll_async", "wl_engine_poll_ready", "wl_engine_retire", "wl_engine_bytes", "wl_pf_force",
+    "wl_engine_step", "wl_engine_run", "wl_engine_poll", "wl_engine_poll_async", "wl_engine_poll_ready", "wl_engine_retire", "wl_engine_bytes", "wl_pf_force", "wl_pf_force_eo",
     "wl_engine_stream", "wl_engine_time_hop", "wl_engine_time_update_hop", "wl_engine_time_cg_hop", "wl_kernel_launches", "wl_engine_debug_apply",
     "wl_apply_schur_normal_noalloc", "wl_gauge_force", "wl_gauge_evolve", "wl_gauge_plaquette_sum",
     "wl_momentum_kinetic", "wl_pion_correlator", "wl_bounds_errors", "wl_random_spinor", "wl_random_algebra",
@@ -108,6 +108,7 @@ def load_library(path: Optional[str] = None) -> ctypes.CDLL:
         "wl_engine_retire": (i, [vp, i, vp, ctypes.POINTER(WLSolveStats)]),
         "wl_engine_bytes": (ctypes.c_int64, [vp, i, i, i]),
         "wl_pf_force": (i, [vp, vp, vp, vp, d, i, vp]),
+        "wl_pf_force_eo": (i, [vp, vp, vp, vp, d, vp, vp]),
         "wl_engine_stream": (vp, [vp]),
         "wl_engine_time_hop": (i, [vp, i, pd, pd]),
         "wl_engine_time_update_hop": (i, [vp, i, pd, pd]),
@@ -274,6 +275,18 @@ class WilsonContext:
         self._check(self.lib.wl_pf_force(self.handle, gauge.handle, _ptr(X), _ptr(Y), float(coef), int(acc),
                                          _ptr(F)))
         return F
+
+    def _force_into(self, gauge: Gauge, X, Y, F, eo_coef: Optional[float] = None):
+        """F = the force of X, Y (pf_force), or with eo_coef the even-odd force of X_e, Y_e times
+        eo_coef; complex128 fields of one configuration on this device, F overwritten."""
+        import torch
+
+        if eo_coef is None:
+            self._check(self.lib.wl_pf_force(self.handle, gauge.handle, _ptr(X), _ptr(Y), 1.0, 0, _ptr(F)))
+            return
+        scratch = torch.empty((2, *self.lattice_shape, 4, 3), dtype=torch.complex128, device=self.device)
+        self._check(self.lib.wl_pf_force_eo(self.handle, gauge.handle, _ptr(X), _ptr(Y), float(eo_coef),
+                                            _ptr(scratch), _ptr(F)))
 
     # ------------------------------------------------------------ gauge sector
     def _links(self, x, name):

@@ -789,7 +789,7 @@ class SU3WilsonNf2(SU3YangMills):
         X, Y = self._as_tensor(X), self._as_tensor(Y)
         F = torch.empty((X.shape[0], 4, *self.lattice_shape, 3, 3), dtype=torch.complex128, device=self.device)
         for b in range(X.shape[0]):
-            F[b] = self.ctx.pf_force(gauges[b], X[b], Y[b])
+            self.ctx._force_into(gauges[b], X[b], Y[b], F[b])
         return self._out(self._from_bm(F))
 
     def eop_pseudofermion_force_from_solution(self, U, X_e, Y_e):
@@ -799,10 +799,7 @@ class SU3WilsonNf2(SU3YangMills):
         X_e, Y_e = self._as_tensor(X_e), self._as_tensor(Y_e)
         F = torch.empty((X_e.shape[0], 4, *self.lattice_shape, 3, 3), dtype=torch.complex128, device=self.device)
         for b in range(X_e.shape[0]):
-            kx = self.ctx.apply("K_OE", gauges[b], self.mass, X_e[b])
-            ky = self.ctx.apply("KDAG_OE", gauges[b], self.mass, Y_e[b])
-            Fb = self.ctx.pf_force(gauges[b], kx, Y_e[b], coef=-alpha)
-            F[b] = self.ctx.pf_force(gauges[b], X_e[b], ky, coef=-alpha, F=Fb)
+            self.ctx._force_into(gauges[b], X_e[b], Y_e[b], F[b], eo_coef=-alpha)
         return self._out(self._from_bm(F))
 
     # ------------------------------------------------------------------ HMC hooks (:1599-1635)
