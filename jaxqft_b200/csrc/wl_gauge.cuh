@@ -11,7 +11,7 @@
 // All FP64.  One thread per link (force, drift, kinetic) or per site (plaquette);
 // sums are deterministic block partials finished by reduce_finalize_kernel.
 #pragma once
-#include "wl_hop.cuh"
+#include "wl_refsite.cuh"
 
 namespace wl {
 
@@ -93,10 +93,12 @@ WL_D void m3_ta(const M3& x, M3& y, double coef) {
     for (int j = 0; j < 3; ++j) y.m[i][j] = coef * y.m[i][j];
 }
 
-// exp(A) by a degree-14 Taylor polynomial (Horner) after scaling A by 2^-s so that
-// its max-row-sum norm is <= 1/2, then s squarings (scaling and squaring, as in
-// Moler and Van Loan, "Nineteen dubious ways to compute the exponential of a
-// matrix", method 3).  Truncation error <= 0.5^15/15! ~ 2e-17 relative.
+// exp(A): the degree-18 Taylor polynomial of a = A 2^-s (max-row-sum norm <= 1, truncation 1/19! ~ 8e-18),
+// squared s times (scaling and squaring, as in Moler and Van Loan, "Nineteen dubious ways to compute the
+// exponential of a matrix", method 3).  The polynomial is evaluated modulo the characteristic polynomial: by
+// Cayley-Hamilton a^3 = t a^2 - m a + d with t = tr a, m = (t^2 - tr a^2) / 2, d = det a, so Horner's rule runs
+// on the three coefficients of q0 + q1 a + q2 a^2 (12 FMAs a step) and one matrix product, a^2, is all that is
+// left of the fourteen products of a matrix Horner scheme.
 WL_D void m3_exp(const M3& A, M3& E) {
   double nrm = 0.0;
 #pragma unroll
@@ -107,35 +109,51 @@ WL_D void m3_exp(const M3& A, M3& E) {
     nrm = fmax(nrm, r);
   }
   int s = 0;
-  while (nrm > 0.5 && s < 64) {  // bounded: at most 64 halvings
+  while (nrm > 1.0 && s < 64) {  // bounded: at most 64 halvings
     nrm *= 0.5;
     ++s;
   }
   const double sc = ldexp(1.0, -s);
-  M3 a;
+  M3 a, a2;
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) a.m[i][j] = sc * A.m[i][j];
-  // E = I + a/1 (I + a/2 (I + ... (I + a/14)))
-  M3 t;
+  m3_mul(a, a, a2);
+  const cplx<double> t = a.m[0][0] + a.m[1][1] + a.m[2][2];
+  const cplx<double> m = 0.5 * (t * t - (a2.m[0][0] + a2.m[1][1] + a2.m[2][2]));
+  const cplx<double> d = a.m[0][0] * (a.m[1][1] * a.m[2][2] - a.m[1][2] * a.m[2][1]) -
+                         a.m[0][1] * (a.m[1][0] * a.m[2][2] - a.m[1][2] * a.m[2][0]) +
+                         a.m[0][2] * (a.m[1][0] * a.m[2][1] - a.m[1][1] * a.m[2][0]);
+  // 1/k!, k = 0..18 (exact quotients rounded by the compiler)
+  constexpr double c[19] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320,
+                            1.0 / 362880, 1.0 / 3628800, 1.0 / 39916800, 1.0 / 479001600, 1.0 / 6227020800.0,
+                            1.0 / 87178291200.0, 1.0 / 1307674368000.0, 1.0 / 20922789888000.0,
+                            1.0 / 355687428096000.0, 1.0 / 6402373705728000.0};
+  cplx<double> q0 = {c[18], 0.0}, q1 = {0.0, 0.0}, q2 = {0.0, 0.0};
+#pragma unroll
+  for (int k = 17; k >= 0; --k) {  // (q0 + q1 a + q2 a^2) a + c_k
+    const cplx<double> p0 = q2 * d, p1 = q2 * m, p2 = q2 * t;
+    q2 = q1 + p2;
+    q1 = q0 - p1;
+    q0 = {c[k] + p0.re, p0.im};
+  }
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) E.m[i][j] = {i == j ? 1.0 : 0.0, 0.0};
+    for (int j = 0; j < 3; ++j) {
+      cplx<double> e = {0.0, 0.0};
+      fma_(e, q2, a2.m[i][j]);
+      fma_(e, q1, a.m[i][j]);
+      E.m[i][j] = i == j ? e + q0 : e;
+    }
+  if (s > 0) {
+    M3 w;
 #pragma unroll 1
-  for (int k = 14; k >= 1; --k) {
-    m3_mul(a, E, t);
-    const double inv = 1.0 / k;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) E.m[i][j] = {(i == j ? 1.0 : 0.0) + inv * t.m[i][j].re, inv * t.m[i][j].im};
-  }
-#pragma unroll 1
-  for (int q = 0; q < s; ++q) {
-    m3_mul(E, E, t);
-    E = t;
+    for (int q = 0; q < s; ++q) {
+      m3_mul(E, E, w);
+      E = w;
+    }
   }
 }
 
@@ -175,63 +193,160 @@ WL_D const double2* glink(const GaugeArgs& A, const double2* base, int b, int mu
   return base + (((long long)b * 4 + mu) * A.g.V + f) * 9;
 }
 
-// grid: x over sites, y = mu, z = batch
-__global__ void __launch_bounds__(128) gauge_force_kernel(GaugeArgs A) {
-  const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int mu = blockIdx.y, b = blockIdx.z;
-  if (f >= A.g.V) return;
-  int x[4];
-  gcoords(A.g, f, x);
-  M3 st, t1, t2, u1, u2, u3;
+// 16-byte asynchronous copy global -> shared, and the wait for all of this thread's copies
+WL_D void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+WL_D void cp16_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+WL_D void m3_lds(M3& a, const double2* p) {
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) st.m[i][j] = {0.0, 0.0};
-#pragma unroll 1
-  for (int nu = 0; nu < 4; ++nu) {
-    if (nu == mu) continue;
-    // forward: U_nu(x) U_mu(x+nu) U_nu(x+mu)^dag
-    m3_load(u1, glink(A, A.U, b, nu, f));
-    m3_load(u2, glink(A, A.U, b, mu, gshift(A.g, x, nu, +1, mu, 0)));
-    m3_load(u3, glink(A, A.U, b, nu, gshift(A.g, x, mu, +1, nu, 0)));
-    m3_mul(u1, u2, t1);
-    m3_mul_nd(t1, u3, t2);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) st.m[i][j] = st.m[i][j] + t2.m[i][j];
-    // backward: U_nu(x-nu)^dag U_mu(x-nu) U_nu(x-nu+mu)
-    const long long fm = gshift(A.g, x, nu, -1, mu, 0);
-    m3_load(u1, glink(A, A.U, b, nu, fm));
-    m3_load(u2, glink(A, A.U, b, mu, fm));
-    m3_load(u3, glink(A, A.U, b, nu, gshift(A.g, x, nu, -1, mu, +1)));
-    m3_mul_dn(u1, u2, t1);
-    m3_mul(t1, u3, t2);
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) st.m[i][j] = st.m[i][j] + t2.m[i][j];
+  for (int k = 0; k < 9; ++k) {
+    const double2 v = p[k];
+    a.m[k / 3][k % 3] = {v.x, v.y};
   }
-  m3_load(u1, glink(A, A.U, b, mu, f));
-  m3_mul_nd(u1, st, t1);  // U_mu(x) V^dag
-  m3_ta(t1, t2, A.coef);
-  m3_store(t2, A.out + (((long long)b * 4 + mu) * A.g.V + f) * 9);
 }
 
-// out = exp(coef * P) U, one thread per link (grid.x over all B*4*V links)
-__global__ void __launch_bounds__(128) gauge_evolve_kernel(GaugeArgs A) {
-  const long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= (long long)A.batch * 4 * A.g.V) return;
-  M3 p, e, u, r;
-  m3_load(p, A.P + l * 9);
+// ---------------------------------------------------------------- force
+// Two kernels.  The links arrive as 144-byte matrices; read in place, a warp's 16-byte load spans 36 lines, and at
+// 171 such loads a link the L1 pipe took the whole 174 us of the kernel this replaced (16^3x32).  So the links are
+// first copied to a matrix-element-major scratch, [batch][mu][9][V] double2, through shared memory (both sides
+// contiguous; 25 us), where the same loads are 512 contiguous bytes.
+//
+// gauge_force_kernel: one thread per link.  A block is 32 consecutive sites with one warp per direction, so that the
+// 76 link reads of a site (31 distinct ones per row) meet in L1.  Bound by the latency of those reads at 12 warps
+// per SM (168 registers: three matrices and the staple sum live) next to 1404 FP64 FMAs a link.
+// Measured at 16^3x32: force and drift together 270 -> 220 us on new links each call (floor 47 us of DRAM, 40 us of
+// FP64); on the same links each call the force takes 25 + 113 us against 174 us.  168 registers (3 blocks) 113 us, 8 warps
+// 139 us, 128 registers (spills) 147 us.  Also measured and not kept: the 31 rows of a 16-site segment staged in
+// shared memory with 18 threads a site (215 us: two phase-locked blocks per SM), 8-site segments (234 us), and 4D
+// site tiles per block (117-152 us).
+__global__ void __launch_bounds__(128) gauge_soa_kernel(const double2* __restrict__ src, double2* __restrict__ dst,
+                                                        int V) {
+  __shared__ double2 sm[4][32 * 9];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int f0 = (int)(blockIdx.x * 4 + warp) * 32;
+  if (f0 >= V) return;  // uniform per warp; only warp barriers below
+  const int n = min(32, V - f0);
+  const size_t plane = (size_t)blockIdx.z * 4 + blockIdx.y;  // (configuration, direction)
+  const double2* s = src + (plane * V + f0) * 9;
+  for (int q = lane; q < n * 9; q += 32) cp16(&sm[warp][q], s + q);
+  cp16_wait();
+  __syncwarp();
+  if (lane < n) {
+    double2* o = dst + plane * 9 * V + f0 + lane;
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int k = 0; k < 9; ++k) o[(size_t)k * V] = sm[warp][lane * 9 + k];
+  }
+}
+
+// element k of the link of direction mu at flat site f: base + (mu * 9 + k) * V + f
+WL_D void m3_load_soa(M3& a, const double2* base, int V, int mu, int f) {
+  const double2* p = base + (size_t)mu * 9 * V + f;
 #pragma unroll
-    for (int j = 0; j < 3; ++j) p.m[i][j] = A.coef * p.m[i][j];
-  m3_exp(p, e);
-  m3_load(u, A.U + l * 9);
-  m3_mul(e, u, r);
-  m3_store(r, A.out + l * 9);
+  for (int k = 0; k < 9; ++k) {
+    const double2 v = ldg(p + (size_t)k * V);
+    a.m[k / 3][k % 3] = {v.x, v.y};
+  }
+}
+
+// A.U: the scratch of gauge_soa_kernel.  grid: x over groups of 32 sites, z = batch
+__global__ void __launch_bounds__(128, 3) gauge_force_kernel(GaugeArgs A) {
+  __shared__ double2 sm[4][32 * 9];
+  const Geom& g = A.g;
+  const int mu = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int f0 = (int)blockIdx.x * 32, f = f0 + lane;
+  const size_t plane = (size_t)blockIdx.z * 4;
+  if (f < g.V) {
+    const double2* S = A.U + plane * 9 * g.V;
+    const Site s = site_of_flat(g, f);
+    const auto at = [&](int mu1, int d1, int mu2, int d2) { return (int)gshift(g, s.x, mu1, d1, mu2, d2); };
+    M3 st, t, u, v;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) st.m[i][j] = {0.0, 0.0};
+#pragma unroll 1
+    for (int n = 1; n < 4; ++n) {
+      const int nu = (mu + n) & 3;
+      // forward: U_nu(x) U_mu(x+nu) U_nu(x+mu)^dag
+      m3_load_soa(u, S, g.V, nu, f);
+      m3_load_soa(v, S, g.V, mu, at(nu, +1, mu, 0));
+      m3_mul(u, v, t);
+      m3_load_soa(u, S, g.V, nu, at(mu, +1, nu, 0));
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) fmac_(st.m[i][j], u.m[j][k], t.m[i][k]);
+      // backward: U_nu(x-nu)^dag U_mu(x-nu) U_nu(x-nu+mu)
+      const int fm = at(nu, -1, mu, 0);
+      m3_load_soa(u, S, g.V, nu, fm);
+      m3_load_soa(v, S, g.V, mu, fm);
+      m3_mul_dn(u, v, t);
+      m3_load_soa(u, S, g.V, nu, at(nu, -1, mu, +1));
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) fma_(st.m[i][j], t.m[i][k], u.m[k][j]);
+    }
+    m3_load_soa(u, S, g.V, mu, f);
+    m3_mul_nd(u, st, t);  // U_mu(x) V^dag
+    m3_ta(t, v, A.coef);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) sm[mu][lane * 9 + k] = make_double2(v.m[k / 3][k % 3].re, v.m[k / 3][k % 3].im);
+  }
+  __syncwarp();
+  double2* out = A.out + ((plane + mu) * g.V + f0) * 9;
+  for (int q = lane; q < 9 * min(32, g.V - f0); q += 32) out[q] = sm[mu][q];
+}
+
+// ---------------------------------------------------------------- drift
+// out = exp(coef * P) U, one thread per link (grid.x over all B*4*V links).  A warp copies the P and U of its 32
+// links to shared memory as two contiguous 4608-byte runs, works from there (144-byte rows: no bank conflicts) and
+// returns the result the same way.  Bound by DRAM (432 bytes a link) next to FP64 arithmetic (about 560 FMAs).
+// The kernel it replaced evaluated a degree-14 matrix Horner scheme (about 2450 FMAs) on 16-byte accesses 144 bytes
+// apart.  Measured at 16^3x32: 95 -> 38 us (226 MB: 35 us at the measured copy rate); 3, 4 or 5 blocks per SM alike.
+constexpr int kEvolveThreads = 128;
+
+__global__ void __launch_bounds__(kEvolveThreads, 4) gauge_evolve_kernel(GaugeArgs A) {
+  __shared__ double2 sm[kEvolveThreads / 32][2][32 * 9];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long l0 = ((long long)blockIdx.x * (kEvolveThreads / 32) + warp) * 32;
+  const long long total = (long long)A.batch * 4 * A.g.V;
+  if (l0 >= total) return;  // uniform per warp; only warp barriers below
+  const int n = (int)min(32LL, total - l0);
+  for (int q = lane; q < n * 9; q += 32) {
+    cp16(&sm[warp][0][q], A.P + l0 * 9 + q);
+    cp16(&sm[warp][1][q], A.U + l0 * 9 + q);
+  }
+  cp16_wait();
+  __syncwarp();
+  if (lane < n) {
+    M3 p, e;
+    m3_lds(p, &sm[warp][0][lane * 9]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) p.m[i][j] = A.coef * p.m[i][j];
+    m3_exp(p, e);
+    m3_lds(p, &sm[warp][1][lane * 9]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        cplx<double> r = {0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) fma_(r, e.m[i][k], p.m[k][j]);
+        sm[warp][0][lane * 9 + i * 3 + j] = make_double2(r.re, r.im);
+      }
+  }
+  __syncwarp();
+  for (int q = lane; q < n * 9; q += 32) A.out[l0 * 9 + q] = sm[warp][0][q];
 }
 
 // per-site plaquette sums (grid: x over sites, z = batch); partials[b][block]

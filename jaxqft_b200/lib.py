@@ -41,7 +41,7 @@ EXPORTS = (
     "wl_gauge_destroy", "wl_apply", "wl_solve", "wl_engine_create", "wl_engine_destroy", "wl_engine_admit",
     "wl_engine_step", "wl_engine_run", "wl_engine_poll", "wl_engine_poll_async", "wl_engine_poll_ready", "wl_engine_retire", "wl_engine_bytes", "wl_pf_force", "wl_pf_force_eo",
     "wl_engine_stream", "wl_engine_time_hop", "wl_engine_time_update_hop", "wl_engine_time_cg_hop", "wl_kernel_launches", "wl_engine_debug_apply",
-    "wl_apply_schur_normal_noalloc", "wl_gauge_force", "wl_gauge_evolve", "wl_gauge_plaquette_sum",
+    "wl_apply_schur_normal_noalloc", "wl_gauge_force", "wl_gauge_force_ws", "wl_gauge_evolve", "wl_gauge_plaquette_sum",
     "wl_momentum_kinetic", "wl_pion_correlator", "wl_bounds_errors", "wl_random_spinor", "wl_random_algebra",
     "wl_field_dots", "wl_field_combine",
 )
@@ -118,6 +118,7 @@ def load_library(path: Optional[str] = None) -> ctypes.CDLL:
         "wl_engine_debug_apply": (i, [vp, i, d, vp, vp]),
         "wl_apply_schur_normal_noalloc": (i, [vp, vp, d, u, vp, vp, i]),
         "wl_gauge_force": (i, [vp, vp, i, d, vp]),
+        "wl_gauge_force_ws": (i, [vp, vp, i, d, vp, vp]),
         "wl_gauge_evolve": (i, [vp, vp, vp, i, d, vp]),
         "wl_gauge_plaquette_sum": (i, [vp, vp, i, pd]),
         "wl_momentum_kinetic": (i, [vp, vp, i, pd]),
@@ -303,7 +304,8 @@ class WilsonContext:
         U, B = self._links(U, "U")
         if out is None:
             out = torch.empty_like(U)
-        self._check(self.lib.wl_gauge_force(self.handle, _ptr(U), B, float(beta), _ptr(out)))
+        scratch = torch.empty_like(U)  # element-major copy of the links, from the caching allocator
+        self._check(self.lib.wl_gauge_force_ws(self.handle, _ptr(U), B, float(beta), _ptr(scratch), _ptr(out)))
         return out
 
     def gauge_evolve(self, dt: float, P, U, out=None):

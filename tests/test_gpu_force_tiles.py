@@ -1,10 +1,10 @@
-"""Pseudofermion force kernel at the sizes where its tiling can go wrong: lattices smaller than, equal to and ragged
-against its 64-site blocks, extents of two (both neighbours the same site), fields that are not 32-byte aligned,
-accumulation, and input fields of the even-odd force with odd sites set.
+"""Force and gauge-sector kernels at the sizes where their tiling can go wrong: rows shorter than, equal to and
+ragged against the 16-site segments of the gauge force and the 64-site blocks of the pseudofermion force, extents
+of two (both neighbours the same site), fields that are not 32-byte aligned, accumulation, in-place drift.
 
-Oracle: the numpy restatement.  Tolerance: every force entry is a sum of fewer than 200 products of numbers of
-order one in FP64, so a relative 2-norm error of 1e-13 leaves a factor of more than two over the worst case
-200 eps."""
+Oracle: the numpy restatement.  Tolerances: every force entry is a sum of fewer than 200 products of numbers of
+order one in FP64, so a relative 2-norm error of 1e-13 leaves a factor of more than four over the worst case
+200 eps; the drift squares s ~ log2 ||dt P|| times, each doubling the relative error of a few eps."""
 
 import numpy as np
 import pytest
@@ -60,3 +60,31 @@ def test_even_odd_force_ignores_odd_input_sites(shape):
     F = th.eop_pseudofermion_force_from_solution(torch.from_numpy(U).cuda(), torch.from_numpy(X).cuda(),
                                                  torch.from_numpy(Y).cuda())
     assert rel(F.cpu().numpy(), ref) < 1e-13
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_gauge_force(shape):
+    U = W.hot_links(np.random.default_rng(5), shape, 2, 0.6)
+    F = WilsonContext(shape).gauge_force(torch.from_numpy(U), 5.6).cpu().numpy()
+    assert rel(F, W.gauge_force(U, 5.6)) < 1e-13
+
+
+@pytest.mark.parametrize("dt", [0.0, 1e-9, 0.2, 0.9, 12.0])
+def test_drift_in_place_and_general_generators(dt):
+    """Momenta that are neither traceless nor anti-Hermitian exercise every coefficient of the characteristic
+    polynomial; the output may be the links or the momenta."""
+    shape = (2, 2, 4, 6)  # 384 links: three full blocks of 128 threads
+    rng = np.random.default_rng(6)
+    U = W.hot_links(rng, shape, 1, 0.4)
+    P = W.algebra_field(rng, shape, 1)
+    if dt < 1.0:
+        P = P + 0.3 * (rng.standard_normal(P.shape) + 1j * rng.standard_normal(P.shape))
+    A = torch.from_numpy(dt * P)
+    ref = (torch.linalg.matrix_exp(A) @ torch.from_numpy(U)).numpy()
+    norm = float(A.abs().sum(-1).max())
+    ctx = WilsonContext(shape)
+    tol = 40 * np.finfo(float).eps * (1.0 + norm)
+    for alias in (None, "U", "P"):
+        u, p = torch.from_numpy(U).cuda(), torch.from_numpy(P).cuda()
+        out = ctx.gauge_evolve(dt, p, u, out={None: None, "U": u, "P": p}[alias])
+        assert rel(out.cpu().numpy(), ref) < tol, alias
