@@ -777,7 +777,7 @@ static bool tile_hop_launch(wl_ctx* ctx, const RefSiteArgs& A) {
 // Site-parallel reference-layout hop (wl_refsite.cuh); parity < 0 targets every site.
 template <bool DAG>
 static bool site_hop(wl_ctx* ctx, wl_gauge* G, const void* in, void* out, const void* self, double a, double b,
-                     int nrhs, int parity) {
+                     int nrhs, int parity, bool zero_other) {
   const Geom& g = ctx->g;
   const int kind = ref_hop_kind();
   if ((kind != 0 && kind != 3) || nrhs > 65535) return false;
@@ -791,10 +791,11 @@ static bool site_hop(wl_ctx* ctx, wl_gauge* G, const void* in, void* out, const 
   A.b = b;
   A.nrhs = nrhs;
   A.parity = parity;
+  A.zero_other = zero_other ? 1 : 0;
   const bool w32 = (((uintptr_t)in | (uintptr_t)out | (uintptr_t)self) & 31) == 0;
   if (kind == 3 && parity < 0 && w32 && tile_hop_launch<DAG>(ctx, A)) return true;
-  const long long n = (parity < 0 ? g.V : g.Vh) * 2LL;  // two threads per target site
-  const dim3 grid((unsigned)((n + kRefSiteBlock - 1) / kRefSiteBlock), nrhs);
+  const int per = parity < 0 ? 16 : 32;  // compact sites per block (of both parities, or of one)
+  const dim3 grid((unsigned)((g.Vh + per - 1) / per), nrhs);
   g_launches++;
   if (w32 && ref_sector_enabled()) ref_pair_kernel<DAG, 4, true><<<grid, kRefSiteBlock, 0, ctx->stream>>>(A);
   else if (w32) ref_pair_kernel<DAG, 4><<<grid, kRefSiteBlock, 0, ctx->stream>>>(A);
@@ -803,10 +804,12 @@ static bool site_hop(wl_ctx* ctx, wl_gauge* G, const void* in, void* out, const 
 }
 
 // out(target parities) = a*self + b*hop(in); npar = 2 for both parities, else target parity0 only
+// (`zero_other`: and zero on the other parity)
 template <bool DAG>
 static void ref_hop(wl_ctx* ctx, wl_gauge* G, const void* in, void* out, const void* self, double a, double b,
-                    int nrhs, int parity0, int npar) {
-  if (site_hop<DAG>(ctx, G, in, out, self, a, b, nrhs, npar == 2 ? -1 : parity0)) return;
+                    int nrhs, int parity0, int npar, bool zero_other = false) {
+  if (site_hop<DAG>(ctx, G, in, out, self, a, b, nrhs, npar == 2 ? -1 : parity0, zero_other)) return;
+  if (zero_other) cudaMemsetAsync(out, 0, (size_t)nrhs * ctx->g.V * 12 * sizeof(double2), ctx->stream);
   if (row_hop<DAG>(ctx, G, in, out, self, a, b, nrhs, npar == 2 ? 3 : (1 << parity0))) return;
   RefHopArgs A = ref_args(ctx, G, in, out, self, a, b, nrhs, parity0);
   Tune t;
@@ -827,7 +830,6 @@ extern "C" wl_status wl_apply(wl_ctx* ctx, wl_gauge* G, int op, double mass, uns
   const double m0 = mass + 4.0;
   const size_t fbytes = (size_t)nrhs * g.V * 12 * sizeof(double2);
   const bool norm = (flags & WL_FLAG_NORMALIZED) != 0;
-  cudaStream_t st = ctx->stream;
   switch (op) {
     case WL_OP_D: ref_hop<false>(ctx, G, in, out, in, m0, -0.5, nrhs, 0, 2); break;
     case WL_OP_DDAG: ref_hop<true>(ctx, G, in, out, in, m0, -0.5, nrhs, 0, 2); break;
@@ -845,9 +847,9 @@ extern "C" wl_status wl_apply(wl_ctx* ctx, wl_gauge* G, int op, double mass, uns
     case WL_OP_KDAG_OE:
     case WL_OP_KDAG_EO: {
       const int target = (op == WL_OP_K_OE || op == WL_OP_KDAG_OE) ? 1 : 0;
-      WL_CUDA(ctx, cudaMemsetAsync(out, 0, fbytes, st));
-      if (op == WL_OP_K_OE || op == WL_OP_K_EO) ref_hop<false>(ctx, G, in, out, nullptr, 0.0, -0.5, nrhs, target, 1);
-      else ref_hop<true>(ctx, G, in, out, nullptr, 0.0, -0.5, nrhs, target, 1);
+      if (op == WL_OP_K_OE || op == WL_OP_K_EO)
+        ref_hop<false>(ctx, G, in, out, nullptr, 0.0, -0.5, nrhs, target, 1, true);
+      else ref_hop<true>(ctx, G, in, out, nullptr, 0.0, -0.5, nrhs, target, 1, true);
       break;
     }
     case WL_OP_SCHUR_E:
@@ -858,15 +860,14 @@ extern "C" wl_status wl_apply(wl_ctx* ctx, wl_gauge* G, int op, double mass, uns
       const bool dag = (op == WL_OP_SCHUR_E_DAG);
       wl_status s = ensure_tmp(ctx, fbytes);
       if (s != WL_OK) return s;
-      WL_CUDA(ctx, cudaMemsetAsync(out, 0, fbytes, st));
       const double c0 = norm ? 1.0 : m0;
       const double c1 = norm ? 0.5 / (m0 * m0) : 0.5 / m0;
       if (dag) {
         ref_hop<true>(ctx, G, in, ctx->tmp, nullptr, 0.0, -0.5, nrhs, 1 - p, 1);
-        ref_hop<true>(ctx, G, ctx->tmp, out, in, c0, c1, nrhs, p, 1);
+        ref_hop<true>(ctx, G, ctx->tmp, out, in, c0, c1, nrhs, p, 1, true);
       } else {
         ref_hop<false>(ctx, G, in, ctx->tmp, nullptr, 0.0, -0.5, nrhs, 1 - p, 1);
-        ref_hop<false>(ctx, G, ctx->tmp, out, in, c0, c1, nrhs, p, 1);
+        ref_hop<false>(ctx, G, ctx->tmp, out, in, c0, c1, nrhs, p, 1, true);
       }
       break;
     }
@@ -876,14 +877,13 @@ extern "C" wl_status wl_apply(wl_ctx* ctx, wl_gauge* G, int op, double mass, uns
       if (s != WL_OK) return s;
       void* t1 = ctx->tmp;
       void* y = (char*)ctx->tmp + fbytes;
-      WL_CUDA(ctx, cudaMemsetAsync(y, 0, fbytes, st));
-      WL_CUDA(ctx, cudaMemsetAsync(out, 0, fbytes, st));
+      // every hop reads one parity of its source, the one its producer wrote
       const double c0 = norm ? 1.0 : m0;
       const double c1 = norm ? 0.5 / (m0 * m0) : 0.5 / m0;
       ref_hop<false>(ctx, G, in, t1, nullptr, 0.0, -0.5, nrhs, 1, 1);
       ref_hop<false>(ctx, G, t1, y, in, c0, c1, nrhs, 0, 1);
       ref_hop<true>(ctx, G, y, t1, nullptr, 0.0, -0.5, nrhs, 1, 1);
-      ref_hop<true>(ctx, G, t1, out, y, c0, c1, nrhs, 0, 1);
+      ref_hop<true>(ctx, G, t1, out, y, c0, c1, nrhs, 0, 1, true);
       break;
     }
     default: WL_FAIL(ctx, WL_ERR_ARG, "unknown operator");
@@ -2740,10 +2740,9 @@ extern "C" wl_status wl_apply_schur_normal_noalloc(wl_ctx* ctx, wl_gauge* G, dou
   const double m0 = mass + 4.0;
   const double c0 = norm ? 1.0 : m0;
   const double c1 = norm ? 0.5 / (m0 * m0) : 0.5 / m0;
-  WL_CUDA(ctx, cudaMemsetAsync(out, 0, fbytes, ctx->stream));  // odd sites of the result are zero
   ref_hop<false>(ctx, G, in, t1, nullptr, 0.0, -0.5, nrhs, 1, 1);
   ref_hop<false>(ctx, G, t1, y, in, c0, c1, nrhs, 0, 1);
   ref_hop<true>(ctx, G, y, t1, nullptr, 0.0, -0.5, nrhs, 1, 1);
-  ref_hop<true>(ctx, G, t1, out, y, c0, c1, nrhs, 0, 1);
+  ref_hop<true>(ctx, G, t1, out, y, c0, c1, nrhs, 0, 1, true);  // odd sites of the result are zero
   return check_launch(ctx, "wl_apply_schur_normal_noalloc");
 }

@@ -12,19 +12,25 @@
 // of every link (forward from x, backward from x + mu) are L2 hits: the reuse
 // distance is at most one x-slice of the lattice (Ly*Lz*Lt sites).
 //
-// Thread mapping: with both parities targeted (D, D^dag, K) pair i of the grid
-// row owns flat site i, so a warp covers 16 consecutive sites; with one target
-// parity p pair i owns compact site i of parity p.
+// Thread mapping: a warp owns 16 consecutive compact sites of one parity, so that each of its link loads is one
+// contiguous 256-byte run.  With both parities targeted (D, D^dag, K) the two warps of a block take the even and
+// the odd sites of the same 32 flat sites, whose neighbours they share in L1; with one target parity p the block
+// takes 32 compact sites of parity p, and with `zero_other` each pair also clears its site's flat neighbour, the
+// other parity's site of the same compact index, so that the masked operators need no separate memset.
 //
 // Contract = row_hop_kernel: out = a*self + b*acc on the target sites,
 //   acc = sum_mu [(1 + cf g_mu) U_mu(x) psi(x+mu) + (1 + cb g_mu) U_mu^dag(x-mu) psi(x-mu)],
 // cf = -1 (D) or +1 (D^dag), cb = -cf, boundary phase on the forward hop from
 // x_mu = L_mu - 1 and (conjugated) on the backward hop into x_mu = 0.
 //
-// Measured at 24^3x48 (1 RHS): 0.217 ms, limited by the L1 data pipe (83-88 % of
-// its wavefront rate at 33 % of DRAM bandwidth): every load instruction of a
-// warp touches one or two sectors of each of its 16 sites.  A one-thread-per-
-// site form (six 32-byte loads per neighbour, 168 registers) timed the same.
+// Bound by the L1 data pipe (79 % of its wavefront rate at 50 % of DRAM bandwidth at 24^3x48): every spinor load of
+// a warp touches one 64-byte piece of each of its 16 sites, and every link is delivered to both threads of a pair.
+// Measured (B200, new buffers each call) against warps of 16 consecutive flat sites, whose link loads are two
+// half-used runs, in blocks of 128 threads with separate memsets: S_e^dag S_e of three fields at 6x10x14x18 51.3 ->
+// 43.0 us, D at 24^3x48 201 -> 198 us, D^dag of 12 fields at 16^3x32 unchanged (415 us), D at 8^4 unchanged.  On the
+// same buffers every call: D at 24^3x48 187 -> 174 us, three fields at 6x10x14x18 19.6 -> 16.8 us.
+// Measured and not kept: 4D site tiles per block (187-227 us at 24^3x48), two to four fields per pair on one link
+// load (376-391 against 393 us for the 12 fields, at 8-12 warps per SM), the four directions on four warps (256 us).
 #pragma once
 #include "wl_hop.cuh"
 
@@ -39,6 +45,7 @@ struct RefSiteArgs {
   double a, b;
   int nrhs;
   int parity;           // target parity, or -1 for every site
+  int zero_other;       // one target parity: store zeros on the other parity's sites
 };
 
 // 32-byte (W = 4) or 16-byte (W = 2) vector accesses of doubles.  The 32-byte
@@ -66,7 +73,7 @@ WL_D void st_vec(double* p, const double* v) {
   }
 }
 
-constexpr int kRefSiteBlock = 128;
+constexpr int kRefSiteBlock = 64;
 
 // ---------------------------------------------------------------- two threads per site
 // Thread j (j = lane & 1) of a pair forms half-spinor row j of every hop (as
@@ -391,33 +398,29 @@ WL_D void refpair_mu(const RefSiteArgs& A, const double* base, const Site& s, in
 }
 
 #ifndef WL_REFPAIR_MINB
-#define WL_REFPAIR_MINB 4  // resident 128-thread blocks per SM the pair kernel is compiled for
+#define WL_REFPAIR_MINB 8  // resident blocks per SM the pair kernel is compiled for (128 registers)
 #endif
 
 template <bool DAG, int W, bool SECT = false>
 __global__ void __launch_bounds__(kRefSiteBlock, WL_REFPAIR_MINB) ref_pair_kernel(RefSiteArgs A) {
   static_assert(!SECT || W == 4, "sector loads use 32-byte vectors");
   const Geom& g = A.g;
-  const int i = blockIdx.x * (blockDim.x >> 1) + (threadIdx.x >> 1);
   const int j = threadIdx.x & 1;
   const double sg = 1.0 - 2.0 * j;
   const int rhs = blockIdx.y;
-  const bool act = i < (A.parity < 0 ? g.V : g.Vh);
+  // compact site of this pair: 16 per warp, the block's two warps on the two parities or on 32 sites of one
+  const int parity = A.parity < 0 ? (int)(threadIdx.x >> 5) : A.parity;
+  const int i = A.parity < 0 ? (int)blockIdx.x * 16 + (int)((threadIdx.x & 31) >> 1)
+                             : (int)blockIdx.x * 32 + (int)(threadIdx.x >> 1);
+  const bool act = i < g.Vh;
   Site s{};
-  int parity = 0;
   cplx<double> Ac[3], Xc[3], Yc[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) Ac[a] = Xc[a] = Yc[a] = {0.0, 0.0};
   const size_t field = (size_t)rhs * g.V * 24;
   const unsigned pm = __ballot_sync(0xffffffffu, act);  // both threads of a pair share `act`
   if (act) {
-    if (A.parity < 0) {  // every site: i is the flat index
-      s = site_of_flat(g, i);
-      parity = (s.x[0] + s.x[1] + s.x[2] + s.x[3]) & 1;
-    } else {  // one parity: i is the compact index
-      parity = A.parity;
-      s = site_from_compact(g, parity, i);
-    }
+    s = site_from_compact(g, parity, i);
     const double* base = A.in + field;
     refpair_mu<0, DAG, W, SECT>(A, base, s, parity, j, sg, pm, Ac, Xc, Yc);
     refpair_mu<1, DAG, W, SECT>(A, base, s, parity, j, sg, pm, Ac, Xc, Yc);
@@ -427,6 +430,12 @@ __global__ void __launch_bounds__(kRefSiteBlock, WL_REFPAIR_MINB) ref_pair_kerne
   const size_t flat = (size_t)s.row * g.L[3] + s.x[3];
   if (SECT) pair_store_sect(A, field + flat * 24, act, j, Ac, Xc, Yc);
   else pair_store<W>(A, field + flat * 24 + 12 * j, act, j, Ac, Xc, Yc);  // this thread's two spins
+  if (act && A.zero_other && A.parity >= 0) {
+    const double z[4] = {0.0, 0.0, 0.0, 0.0};
+    double* o = A.out + field + (flat ^ 1) * 24;
+#pragma unroll
+    for (int k = 0; k < 24; k += 2 * W) st_vec<W>(o + k + W * j, z);
+  }
 }
 
 }  // namespace wl
