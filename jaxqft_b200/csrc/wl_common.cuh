@@ -193,8 +193,10 @@ WL_D unsigned int f2h(float a, float b) {
 // ---------------------------------------------------------------- precisions
 enum Prec { P_DOUBLE = 0, P_SINGLE = 1, P_HALF = 2 };
 
-// Spinor field in the internal SoA compact layout.
-template <int P> struct SpinorField;
+// Spinor field in the internal SoA compact layout.  NC: loads go through the read-only path (ld.global.nc), which a
+// kernel may use for fields that no block of the launch writes; NC = false makes every load an ordinary one, for the
+// persistent iteration kernel, whose phases read what other blocks wrote before a grid barrier.
+template <int P, bool NC = true> struct SpinorField;
 
 // Element (rhs, chunk k, site c) lives at ptr[rhs*rstride + k*kstride + c*cstride]
 // (chunk = 16 bytes).  Two layouts use this accessor:
@@ -212,14 +214,15 @@ struct Strides {
   WL_D unsigned nat(int rhs, unsigned c) const { return rhs * nrstride + c * ncstride; }
 };
 
-template <> struct SpinorField<P_DOUBLE> : Strides {
+template <bool NC> struct SpinorField<P_DOUBLE, NC> : Strides {
   using real = double;
+  template <class V> WL_D static V ld(const V* p) { return NC ? ldg(p) : *p; }
   double2* ptr;
   float* norm;  // unused
   WL_D void load(Spinor<double>& s, int rhs, long long c) const {
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      double2 v = ldg(ptr + at(rhs, k, c));
+      double2 v = ld(ptr + at(rhs, k, c));
       s.v[k / 3][k % 3] = {v.x, v.y};
     }
   }
@@ -236,21 +239,22 @@ template <> struct SpinorField<P_DOUBLE> : Strides {
   }
 };
 
-template <> struct SpinorField<P_SINGLE> : Strides {
+template <bool NC> struct SpinorField<P_SINGLE, NC> : Strides {
   using real = float;
+  template <class V> WL_D static V ld(const V* p) { return NC ? ldg(p) : *p; }
   float4* ptr;
   float* norm;
-  template <bool NC>
+  template <bool RO>
   WL_D void load_impl(Spinor<float>& s, int rhs, long long c) const {
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      float4 v = NC ? ldg(ptr + at(rhs, k, c)) : ptr[at(rhs, k, c)];
+      float4 v = RO ? ldg(ptr + at(rhs, k, c)) : ptr[at(rhs, k, c)];
       int i0 = 2 * k, i1 = 2 * k + 1;
       s.v[i0 / 3][i0 % 3] = {v.x, v.y};
       s.v[i1 / 3][i1 % 3] = {v.z, v.w};
     }
   }
-  WL_D void load(Spinor<float>& s, int rhs, long long c) const { load_impl<true>(s, rhs, c); }
+  WL_D void load(Spinor<float>& s, int rhs, long long c) const { load_impl<NC>(s, rhs, c); }
   WL_D void load_plain(Spinor<float>& s, int rhs, long long c) const { load_impl<false>(s, rhs, c); }
   WL_D void store(const Spinor<float>& s, int rhs, long long c) const {
 #pragma unroll
@@ -266,16 +270,17 @@ template <> struct SpinorField<P_SINGLE> : Strides {
 // the four spins as half2 (re, im), plus one float norm (value = norm * half).
 // The colour-major order lets the tensor-core hop give each lane of an MMA
 // group one colour of all four spins with a single 16-byte load.
-template <> struct SpinorField<P_HALF> : Strides {
+template <bool NC> struct SpinorField<P_HALF, NC> : Strides {
   using real = float;
+  template <class V> WL_D static V ld(const V* p) { return NC ? ldg(p) : *p; }
   uint4* ptr;
   float* norm;
-  template <bool NC>
+  template <bool RO>
   WL_D void load_impl(Spinor<float>& s, int rhs, long long c) const {
-    float nrm = NC ? ldg(norm + nat(rhs, c)) : norm[nat(rhs, c)];
+    float nrm = RO ? ldg(norm + nat(rhs, c)) : norm[nat(rhs, c)];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {  // chunk k = colour k, spins 0..3
-      uint4 v = NC ? ldg(ptr + at(rhs, k, c)) : ptr[at(rhs, k, c)];
+      uint4 v = RO ? ldg(ptr + at(rhs, k, c)) : ptr[at(rhs, k, c)];
       float2 a0 = h2f(v.x), a1 = h2f(v.y), a2 = h2f(v.z), a3 = h2f(v.w);
       s.v[0][k] = {a0.x * nrm, a0.y * nrm};
       s.v[1][k] = {a1.x * nrm, a1.y * nrm};
@@ -283,7 +288,7 @@ template <> struct SpinorField<P_HALF> : Strides {
       s.v[3][k] = {a3.x * nrm, a3.y * nrm};
     }
   }
-  WL_D void load(Spinor<float>& s, int rhs, long long c) const { load_impl<true>(s, rhs, c); }
+  WL_D void load(Spinor<float>& s, int rhs, long long c) const { load_impl<NC>(s, rhs, c); }
   WL_D void load_plain(Spinor<float>& s, int rhs, long long c) const { load_impl<false>(s, rhs, c); }
   WL_D void store(const Spinor<float>& s, int rhs, long long c) const {
     float mx = 0.f;
@@ -326,28 +331,28 @@ WL_D float2 fmul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 // store: v = values; FP16 stores pick the per-site norm max|v| and pack pairs
 template <class SF> struct Packed;
 
-template <> struct Packed<SpinorField<P_SINGLE>> {
-  WL_D static float load(const SpinorField<P_SINGLE>& f, int rhs, unsigned c, float2 (&v)[12]) {
+template <bool NC> struct Packed<SpinorField<P_SINGLE, NC>> {
+  WL_D static float load(const SpinorField<P_SINGLE, NC>& f, int rhs, unsigned c, float2 (&v)[12]) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      const float4 q = ldg(f.ptr + f.at(rhs, k, c));
+      const float4 q = f.ld(f.ptr + f.at(rhs, k, c));
       v[2 * k] = f2(q.x, q.y);
       v[2 * k + 1] = f2(q.z, q.w);
     }
     return 1.0f;
   }
-  WL_D static void store(const SpinorField<P_SINGLE>& f, int rhs, unsigned c, const float2 (&v)[12]) {
+  WL_D static void store(const SpinorField<P_SINGLE, NC>& f, int rhs, unsigned c, const float2 (&v)[12]) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) f.ptr[f.at(rhs, k, c)] = make_float4(v[2 * k].x, v[2 * k].y, v[2 * k + 1].x, v[2 * k + 1].y);
   }
 };
 
-template <> struct Packed<SpinorField<P_HALF>> {
-  WL_D static float load(const SpinorField<P_HALF>& f, int rhs, unsigned c, float2 (&v)[12]) {
-    const float n = ldg(f.norm + f.nat(rhs, c));
+template <bool NC> struct Packed<SpinorField<P_HALF, NC>> {
+  WL_D static float load(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, float2 (&v)[12]) {
+    const float n = f.ld(f.norm + f.nat(rhs, c));
 #pragma unroll
     for (int k = 0; k < 3; ++k) {  // chunk k = colour k, spins 0..3
-      const uint4 q = ldg(f.ptr + f.at(rhs, k, c));
+      const uint4 q = f.ld(f.ptr + f.at(rhs, k, c));
       v[k] = h2f(q.x);
       v[3 + k] = h2f(q.y);
       v[6 + k] = h2f(q.z);
@@ -355,7 +360,7 @@ template <> struct Packed<SpinorField<P_HALF>> {
     }
     return n;
   }
-  WL_D static void store(const SpinorField<P_HALF>& f, int rhs, unsigned c, const float2 (&v)[12]) {
+  WL_D static void store(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, const float2 (&v)[12]) {
     float mx = 0.f;
 #pragma unroll
     for (int k = 0; k < 12; ++k) mx = fmaxf(mx, fmaxf(fabsf(v[k].x), fabsf(v[k].y)));

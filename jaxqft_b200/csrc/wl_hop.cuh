@@ -308,19 +308,21 @@ __global__ void __launch_bounds__(256) hop_kernel(HopArgs<LF, SF, EPI> A) {
 // Spin s (three colours) of an FP32 record: complex z = 3 s + colour sits in
 // 16-byte chunk z / 2 (half z % 2), so spin s is chunk (3 s - (s & 1)) / 2 from
 // colour 0 (even s: the whole chunk; odd s: its upper half) and the next chunk.
-WL_D void pair_spin_load(const SpinorField<P_SINGLE>& f, int rhs, unsigned c, int s, cplx<float> (&v)[3]) {
+template <bool NC>
+WL_D void pair_spin_load(const SpinorField<P_SINGLE, NC>& f, int rhs, unsigned c, int s, cplx<float> (&v)[3]) {
   const int odd = s & 1;
   const int k0 = (3 * s - odd) >> 1;
-  const float4 q0 = ldg(f.ptr + f.at(rhs, k0, c));
-  const float4 q1 = ldg(f.ptr + f.at(rhs, k0 + 1, c));
+  const float4 q0 = f.ld(f.ptr + f.at(rhs, k0, c));
+  const float4 q1 = f.ld(f.ptr + f.at(rhs, k0 + 1, c));
   v[0] = odd ? cplx<float>{q0.z, q0.w} : cplx<float>{q0.x, q0.y};
   v[1] = odd ? cplx<float>{q1.x, q1.y} : cplx<float>{q0.z, q0.w};
   v[2] = odd ? cplx<float>{q1.z, q1.w} : cplx<float>{q1.x, q1.y};
 }
-WL_D void pair_spin_load(const SpinorField<P_DOUBLE>& f, int rhs, unsigned c, int s, cplx<double> (&v)[3]) {
+template <bool NC>
+WL_D void pair_spin_load(const SpinorField<P_DOUBLE, NC>& f, int rhs, unsigned c, int s, cplx<double> (&v)[3]) {
 #pragma unroll
   for (int col = 0; col < 3; ++col) {
-    const double2 a = ldg(f.ptr + f.at(rhs, s * 3 + col, c));
+    const double2 a = f.ld(f.ptr + f.at(rhs, s * 3 + col, c));
     v[col] = {a.x, a.y};
   }
 }
@@ -424,9 +426,34 @@ WL_D cplx<T> shfl_pair(cplx<T> v) {
 template <class SF> struct PairMinBlocks {
   static constexpr int value = WL_HOP_PAIR_MINB;
 };
-template <> struct PairMinBlocks<SpinorField<P_SINGLE>> {
+template <bool NC> struct PairMinBlocks<SpinorField<P_SINGLE, NC>> {
   static constexpr int value = WL_HOP_PAIR_MINB_S;
 };
+
+// The stencil of site s for thread j of its pair; on return o[0], o[1] are spins 2j, 2j + 1 of the sum (the
+// xor-shuffle exchange a0 = A_0, a1 = A_1, a2 = Y_0 + X_1, a3 = X_0 + Y_1, subscript = thread of the pair: round 1
+// thread 0 sends X_0 and receives A_1, round 2 thread 0 sends Y_0).  Every lane of the warp must call it.
+template <bool DAG, class LF, class SF, typename T>
+WL_D void pair_stencil(const Geom& g, const LF& links, const SF& src, int parity, const Site& s, int rhs, int j,
+                       bool act, cplx<T> (&o)[2][3]) {
+  const T sg = T(1) - T(2) * T(j);
+  cplx<T> Ac[3], Xc[3], Yc[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) Ac[a] = Xc[a] = Yc[a] = {T(0), T(0)};
+  if (act) {
+    pair_dir<0, DAG>(g, links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
+    pair_dir<1, DAG>(g, links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
+    pair_dir<2, DAG>(g, links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
+    pair_dir<3, DAG>(g, links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const cplx<T> r1 = shfl_pair(j == 0 ? Xc[a] : Ac[a]);
+    const cplx<T> r2 = shfl_pair(Yc[a]);
+    o[0][a] = j == 0 ? Ac[a] : r2 + Xc[a];
+    o[1][a] = j == 0 ? r1 : r1 + Yc[a];
+  }
+}
 
 template <bool DAG, class LF, class SF, class EPI>
 __global__ void __launch_bounds__(256, PairMinBlocks<SF>::value) hop_pair_kernel(HopArgs<LF, SF, EPI> A) {
@@ -434,35 +461,87 @@ __global__ void __launch_bounds__(256, PairMinBlocks<SF>::value) hop_pair_kernel
   static_assert(std::is_same<T, typename LF::real>::value, "links and spinors in the same arithmetic");
   const int c = blockIdx.x * (blockDim.x >> 1) + (threadIdx.x >> 1);
   const int j = threadIdx.x & 1;
-  const T sg = T(1) - T(2) * T(j);
   const int parity = A.parity0 ^ blockIdx.z;
   const int rhs = blockIdx.y;
   const bool act = c < A.g.Vh && rhs < A.nrhs && (A.mask == nullptr || A.mask[rhs] != 0);
-  cplx<T> Ac[3], Xc[3], Yc[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) Ac[a] = Xc[a] = Yc[a] = {T(0), T(0)};
   Site s{};
-  if (act) {
-    s = site_from_compact(A.g, parity, c);
-    const SF& src = A.src[1 - parity];
-    pair_dir<0, DAG>(A.g, A.links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
-    pair_dir<1, DAG>(A.g, A.links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
-    pair_dir<2, DAG>(A.g, A.links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
-    pair_dir<3, DAG>(A.g, A.links, src, parity, s, rhs, j, sg, Ac, Xc, Yc);
-  }
-  // thread 0 of the pair: a0 = A, a1 = A', a2 = Y + X', a3 = X + Y'
-  Spinor<T> acc;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const cplx<T> Ap = shfl_pair(Ac[a]), Xp = shfl_pair(Xc[a]), Yp = shfl_pair(Yc[a]);
-    acc.v[0][a] = Ac[a];
-    acc.v[1][a] = Ap;
-    acc.v[2][a] = Yc[a] + Xp;
-    acc.v[3][a] = Xc[a] + Yp;
-  }
-  double red[1] = {0.0};
-  if (act && j == 0) red[0] = A.epi(rhs, parity, s.c, acc);
+  if (act) s = site_from_compact(A.g, parity, c);
+  cplx<T> o[2][3];
+  pair_stencil<DAG>(A.g, A.links, A.src[1 - parity], parity, s, rhs, j, act, o);
+  double red[1] = {A.epi.half(rhs, parity, (unsigned)s.c, j, act, o)};
   if (EPI::kReduce) reduce_rhs<1>(red, A.red, A.nrhs, A.mask);
+}
+
+// ------------------------------------------------------------------ half sites
+// Spins 2j, 2j + 1 of a site, for the pair kernel's epilogues: both threads of a pair run the epilogue, each on its
+// two spins, so that every field access of a warp uses all lanes and an epilogue's loads are issued twice as wide.
+// (With thread 0 running it alone, the FP64 CG hop at 12^3x24 took 28.8 us of which the stencil is 15.6.)
+template <bool NC>
+WL_D void half_load(const SpinorField<P_DOUBLE, NC>& f, int rhs, unsigned c, int j, cplx<double> (&v)[2][3]) {
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double2 q = f.ld(f.ptr + f.at(rhs, 6 * j + k, c));
+    v[k / 3][k % 3] = {q.x, q.y};
+  }
+}
+template <bool NC>
+WL_D void half_load(const SpinorField<P_SINGLE, NC>& f, int rhs, unsigned c, int j, cplx<float> (&v)[2][3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {  // complex values 6 j + 2 k, 6 j + 2 k + 1
+    const float4 q = f.ld(f.ptr + f.at(rhs, 3 * j + k, c));
+    v[(2 * k) / 3][(2 * k) % 3] = {q.x, q.y};
+    v[(2 * k + 1) / 3][(2 * k + 1) % 3] = {q.z, q.w};
+  }
+}
+// Stores: every lane of the warp calls (the FP16 record's norm is the maximum over the pair); only active ones write.
+template <bool NC>
+WL_D void half_store(const SpinorField<P_DOUBLE, NC>& f, int rhs, unsigned c, int j, bool act,
+                     const cplx<double> (&v)[2][3]) {
+  if (!act) return;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) f.ptr[f.at(rhs, 6 * j + k, c)] = make_double2(v[k / 3][k % 3].re, v[k / 3][k % 3].im);
+}
+template <bool NC>
+WL_D void half_store(const SpinorField<P_SINGLE, NC>& f, int rhs, unsigned c, int j, bool act,
+                     const cplx<float> (&v)[2][3]) {
+  if (!act) return;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const cplx<float> a = v[(2 * k) / 3][(2 * k) % 3], b = v[(2 * k + 1) / 3][(2 * k + 1) % 3];
+    f.ptr[f.at(rhs, 3 * j + k, c)] = make_float4(a.re, a.im, b.re, b.im);
+  }
+}
+template <bool NC>
+WL_D void half_store(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, int j, bool act,
+                     const cplx<float> (&v)[2][3]) {
+  float mx = 0.f;
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) mx = fmaxf(mx, fmaxf(fabsf(v[s][k].re), fabsf(v[s][k].im)));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  if (!act) return;
+  // below FLT_MIN the site is stored as zero (1/mx would overflow, 0 * Inf = NaN)
+  const bool keep = mx >= 1.17549435e-38f;
+  const float inv = keep ? 1.0f / mx : 0.f;
+  if (j == 0) f.norm[f.nat(rhs, c)] = keep ? mx : 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {  // chunk k = colour k; spins 2j, 2j + 1 are its half j
+    uint2 q;
+    q.x = f2h(v[0][k].re * inv, v[0][k].im * inv);
+    q.y = f2h(v[1][k].re * inv, v[1][k].im * inv);
+    reinterpret_cast<uint2*>(f.ptr + f.at(rhs, k, c))[j] = q;
+  }
+}
+
+template <typename T>
+WL_D double hnorm2(const cplx<T> (&v)[2][3]) {
+  double n = 0.0;
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) n += (double)norm2(v[s][c]);
+  return n;
 }
 
 // ------------------------------------------------------------------ epilogues
@@ -511,6 +590,25 @@ struct EpiXpay {
     }
     out[parity].store(o, rhs, idx);
     return RED ? snorm2(o) : 0.0;
+  }
+  // same on the two spins of thread j of a pair (hop_pair_kernel); every lane of the warp calls
+  WL_D double half(int rhs, int parity, unsigned idx, int j, bool act, cplx<typename SF::real> (&acc)[2][3]) const {
+    using T = typename SF::real;
+    if (act) {
+      const T bb = T(b ? b[rhs] : b0);
+      cplx<T> x[2][3];
+      T aa = T(0);
+      if (has_self) {
+        half_load(self[parity], rhs, idx, j, x);
+        aa = T(a ? a[rhs] : a0);
+      }
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[s][c] = has_self ? aa * x[s][c] + bb * acc[s][c] : bb * acc[s][c];
+    }
+    half_store(out[parity], rhs, idx, j, act, acc);
+    return RED && act ? hnorm2(acc) : 0.0;
   }
   // same on packed FP32 pairs (FP16/FP32 fields, RHS-in-lanes kernels)
   WL_D double packed(int rhs, int parity, unsigned idx, float2 (&acc)[12]) const {

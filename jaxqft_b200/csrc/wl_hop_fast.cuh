@@ -11,14 +11,17 @@
 
 namespace wl {
 
+template <class SF> struct IsHalf : std::false_type {};
+template <bool NC> struct IsHalf<SpinorField<P_HALF, NC>> : std::true_type {};
+
 // Raw spinor load: values without the FP16 per-site norm (returned separately).
 template <class SF> struct RawLoad;
 
-template <> struct RawLoad<SpinorField<P_SINGLE>> {
-  WL_D static float load(const SpinorField<P_SINGLE>& f, int rhs, long long c, float2 (&s)[12]) {
+template <bool NC> struct RawLoad<SpinorField<P_SINGLE, NC>> {
+  WL_D static float load(const SpinorField<P_SINGLE, NC>& f, int rhs, long long c, float2 (&s)[12]) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      float4 v = ldg(f.ptr + f.at(rhs, k, c));
+      float4 v = f.ld(f.ptr + f.at(rhs, k, c));
       s[2 * k] = f2(v.x, v.y);
       s[2 * k + 1] = f2(v.z, v.w);
     }
@@ -26,12 +29,12 @@ template <> struct RawLoad<SpinorField<P_SINGLE>> {
   }
 };
 
-template <> struct RawLoad<SpinorField<P_HALF>> {
-  WL_D static float load(const SpinorField<P_HALF>& f, int rhs, long long c, float2 (&s)[12]) {
-    const float n = ldg(f.norm + f.nat(rhs, c));
+template <bool NC> struct RawLoad<SpinorField<P_HALF, NC>> {
+  WL_D static float load(const SpinorField<P_HALF, NC>& f, int rhs, long long c, float2 (&s)[12]) {
+    const float n = f.ld(f.norm + f.nat(rhs, c));
 #pragma unroll
     for (int k = 0; k < 3; ++k) {  // chunk k = colour k, spins 0..3
-      uint4 v = ldg(f.ptr + f.at(rhs, k, c));
+      uint4 v = f.ld(f.ptr + f.at(rhs, k, c));
       s[k] = h2f(v.x);
       s[3 + k] = h2f(v.y);
       s[6 + k] = h2f(v.z);
@@ -344,17 +347,17 @@ WL_D __half2 as_h2(unsigned int u) { return *reinterpret_cast<__half2*>(&u); }
 
 // s[spin*3 + colour] of an FP16 record; for mu = 3 the projector keeps two spins
 // (0, 1 for C > 0, else 2, 3), so only those 8 bytes of each colour chunk are loaded.
-template <int MU, int C>
-WL_D void load_half_spins(const SpinorField<P_HALF>& f, int rhs, unsigned c, __half2 (&s)[12]) {
+template <int MU, int C, bool NC>
+WL_D void load_half_spins(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, __half2 (&s)[12]) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     if (MU == 3) {
       const uint2* q = reinterpret_cast<const uint2*>(f.ptr + f.at(rhs, k, c)) + (C > 0 ? 0 : 1);
-      const uint2 v = __ldg(q);
+      const uint2 v = f.ld(q);
       s[(C > 0 ? 0 : 6) + k] = as_h2(v.x);
       s[(C > 0 ? 3 : 9) + k] = as_h2(v.y);
     } else {
-      const uint4 v = ldg(f.ptr + f.at(rhs, k, c));
+      const uint4 v = f.ld(f.ptr + f.at(rhs, k, c));
       s[k] = as_h2(v.x);
       s[3 + k] = as_h2(v.y);
       s[6 + k] = as_h2(v.z);
@@ -364,19 +367,19 @@ WL_D void load_half_spins(const SpinorField<P_HALF>& f, int rhs, unsigned c, __h
 }
 
 // the projection as half2 values (rows 0, 1 x colours), no conversion and no norm
-template <int MU, int C>
-WL_D void load_project_half2_raw(const SpinorField<P_HALF>& f, int rhs, unsigned c, __half2 (&h)[6]);
+template <int MU, int C, bool NC>
+WL_D void load_project_half2_raw(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, __half2 (&h)[6]);
 
 // the projection as half2 values (rows 0, 1 x colours), no conversion; returns the site norm
-template <int MU, int C>
-WL_D float load_project_half2(const SpinorField<P_HALF>& f, int rhs, unsigned c, __half2 (&h)[6]) {
-  const float n = ldg(f.norm + f.nat(rhs, c));
+template <int MU, int C, bool NC>
+WL_D float load_project_half2(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, __half2 (&h)[6]) {
+  const float n = f.ld(f.norm + f.nat(rhs, c));
   load_project_half2_raw<MU, C>(f, rhs, c, h);
   return n;
 }
 
-template <int MU, int C>
-WL_D void load_project_half2_raw(const SpinorField<P_HALF>& f, int rhs, unsigned c, __half2 (&h)[6]) {
+template <int MU, int C, bool NC>
+WL_D void load_project_half2_raw(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, __half2 (&h)[6]) {
   __half2 s[12];
   load_half_spins<MU, C>(f, rhs, c, s);
   const __half2 pcm = __floats2half2_rn((float)C, -(float)C);  // -iC x = pcm * swap(x)
@@ -400,9 +403,9 @@ WL_D void load_project_half2_raw(const SpinorField<P_HALF>& f, int rhs, unsigned
   }
 }
 
-template <int MU, int C>
-WL_D float load_project_half(const SpinorField<P_HALF>& f, int rhs, unsigned c, float2 (&h)[6]) {
-  const float n = ldg(f.norm + f.nat(rhs, c));
+template <int MU, int C, bool NC>
+WL_D float load_project_half(const SpinorField<P_HALF, NC>& f, int rhs, unsigned c, float2 (&h)[6]) {
+  const float n = f.ld(f.norm + f.nat(rhs, c));
   __half2 s[12];
   load_half_spins<MU, C>(f, rhs, c, s);
   const __half2 pcm = __floats2half2_rn((float)C, -(float)C);  // -iC x = pcm * swap(x)
@@ -435,7 +438,7 @@ WL_D void lane_dir(const SF& src, const LinkSmem* Ls, const int* nbs, int rhs, f
   constexpr int CF = DAG ? +1 : -1;
   constexpr int CB = -CF;
   constexpr float W3 = (MU == 3) ? 2.0f : 1.0f;
-  constexpr bool kHalfProject = WL_HALF_PROJECT && std::is_same<SF, SpinorField<P_HALF>>::value;
+  constexpr bool kHalfProject = WL_HALF_PROJECT && IsHalf<SF>::value;
 #pragma unroll
   for (int dir = 0; dir < 2; ++dir) {
     const int q = 2 * MU + dir;
@@ -508,8 +511,8 @@ WL_D void color_mul_half(const LinkSmem& L, const __half2 (&h)[6], float2 (&uh)[
 }
 
 // Ls: the site's LinkSmem slots; a hop's FP16 pairs sit at the start of its slot
-template <int MU, bool DAG>
-WL_D void lane_dir_hc(const SpinorField<P_HALF>& src, const LinkSmem* Ls, const int* nbs, int rhs,
+template <int MU, bool DAG, bool NC>
+WL_D void lane_dir_hc(const SpinorField<P_HALF, NC>& src, const LinkSmem* Ls, const int* nbs, int rhs,
                       float2 (&acc)[12]) {
   constexpr int CF = DAG ? +1 : -1;
   constexpr int CB = -CF;
@@ -597,8 +600,8 @@ WL_D void accum2_hh(__half2 (&acc)[12], const __half2 (&uh)[6], float w) {
 }
 
 // w[q]: the relative weights of the site's eight neighbours for this RHS
-template <int MU, bool DAG>
-WL_D void lane_dir_hh(const SpinorField<P_HALF>& src, const LinkSmem* Ls, const int* nbs, int rhs,
+template <int MU, bool DAG, bool NC>
+WL_D void lane_dir_hh(const SpinorField<P_HALF, NC>& src, const LinkSmem* Ls, const int* nbs, int rhs,
                       const float (&w)[8], __half2 (&acc)[12]) {
   constexpr int CF = DAG ? +1 : -1;
   constexpr int CB = -CF;
@@ -620,12 +623,12 @@ WL_D void lane_dir_hh(const SpinorField<P_HALF>& src, const LinkSmem* Ls, const 
 }
 
 // The whole stencil of one (site, RHS) with FP16 accumulation; acc = FP32 result.
-template <bool DAG>
-WL_D void lane_site_hh(const SpinorField<P_HALF>& src, const LinkSmem* Ls, const int* nbs, int rhs,
+template <bool DAG, bool NC>
+WL_D void lane_site_hh(const SpinorField<P_HALF, NC>& src, const LinkSmem* Ls, const int* nbs, int rhs,
                        float2 (&acc)[12]) {
   float w[8];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) w[q] = ldg(src.norm + src.nat(rhs, (unsigned)nbs[q]));
+  for (int q = 0; q < 8; ++q) w[q] = src.ld(src.norm + src.nat(rhs, (unsigned)nbs[q]));
   float m = 0.f;
 #pragma unroll
   for (int q = 0; q < 8; ++q) m = fmaxf(m, w[q]);
@@ -681,6 +684,24 @@ WL_D int stage_link(const Geom& g, const LF& links, int parity, int c, int mu, i
   return nb;
 }
 
+// The stencil of one (site, RHS) from staged links: acc (zero on entry) = sum of the eight contributions.
+template <bool DAG, bool HC, bool HA, class SF>
+WL_D void lane_stencil(const SF& src, const LinkSmem* Ls, const int* nbs, int rhs, float2 (&acc)[12]) {
+  if constexpr (HA) {
+    lane_site_hh<DAG>(src, Ls, nbs, rhs, acc);
+  } else if constexpr (HC) {
+    lane_dir_hc<0, DAG>(src, Ls, nbs, rhs, acc);
+    lane_dir_hc<1, DAG>(src, Ls, nbs, rhs, acc);
+    lane_dir_hc<2, DAG>(src, Ls, nbs, rhs, acc);
+    lane_dir_hc<3, DAG>(src, Ls, nbs, rhs, acc);
+  } else {
+    lane_dir<0, DAG>(src, Ls, nbs, rhs, acc);
+    lane_dir<1, DAG>(src, Ls, nbs, rhs, acc);
+    lane_dir<2, DAG>(src, Ls, nbs, rhs, acc);
+    lane_dir<3, DAG>(src, Ls, nbs, rhs, acc);
+  }
+}
+
 // Per-block partial sums: xor-shuffles over the sites of a warp leave lanes
 // 0..R-1 with the warp's sum for RHS rbase + lane; after one barrier threads
 // 0..R-1 add the block's warps in a fixed order and block b writes
@@ -712,7 +733,7 @@ WL_D void reduce_lanes(double v, const Reduce& Rd, int nrhs, const int* /*mask*/
 template <bool DAG, int R, class LF, class SF, class EPI, bool HC = false, bool HA = false>
 __global__ void __launch_bounds__(kLaneBlock, HA ? WL_LANE_MIN_BLOCKS_HA : LaneMinBlocks<DAG, EPI>::value)
     hop_lanes_kernel(HopArgs<LF, SF, EPI> A) {
-  static_assert(!HC || std::is_same<SF, SpinorField<P_HALF>>::value, "FP16 colour multiply needs FP16 fields");
+  static_assert(!HC || IsHalf<SF>::value, "FP16 colour multiply needs FP16 fields");
   static_assert(!HA || HC, "FP16 accumulation runs behind the FP16 colour multiply");
   constexpr int S = kLaneBlock / R;
   __shared__ LaneSmem<R> sm;
@@ -747,21 +768,7 @@ __global__ void __launch_bounds__(kLaneBlock, HA ? WL_LANE_MIN_BLOCKS_HA : LaneM
     for (int k = 0; k < 12; ++k) acc[k] = f2(0.f, 0.f);
     const SF& src = A.src[1 - parity];
     const int* nbs = sm.nb[sl];
-    if constexpr (HA) {
-      lane_site_hh<DAG>(src, sm.link[sl].l, nbs, rhs, acc);
-    } else if constexpr (HC) {
-      const LinkSmem* Ls = sm.link[sl].l;
-      lane_dir_hc<0, DAG>(src, Ls, nbs, rhs, acc);
-      lane_dir_hc<1, DAG>(src, Ls, nbs, rhs, acc);
-      lane_dir_hc<2, DAG>(src, Ls, nbs, rhs, acc);
-      lane_dir_hc<3, DAG>(src, Ls, nbs, rhs, acc);
-    } else {
-      const LinkSmem* Ls = sm.link[sl].l;
-      lane_dir<0, DAG>(src, Ls, nbs, rhs, acc);
-      lane_dir<1, DAG>(src, Ls, nbs, rhs, acc);
-      lane_dir<2, DAG>(src, Ls, nbs, rhs, acc);
-      lane_dir<3, DAG>(src, Ls, nbs, rhs, acc);
-    }
+    lane_stencil<DAG, HC, HA>(src, sm.link[sl].l, nbs, rhs, acc);
     red = A.epi.packed(rhs, parity, (unsigned)c, acc);
   }
   if (EPI::kReduce) reduce_lanes<R>(red, A.red, A.nrhs, A.mask);
@@ -805,7 +812,7 @@ WL_D void load_project_d(const SpinorField<P_DOUBLE>& f, int rhs, unsigned nb, H
 #pragma unroll
   for (int sp = s_lo; sp < s_hi; ++sp)
 #pragma unroll
-    for (int col = 0; col < 3; ++col) v[sp][col] = ldg(f.ptr + f.at(rhs, sp * 3 + col, nb));
+    for (int col = 0; col < 3; ++col) v[sp][col] = f.ld(f.ptr + f.at(rhs, sp * 3 + col, nb));
 #pragma unroll
   for (int col = 0; col < 3; ++col) {
     if (MU == 3) {

@@ -222,6 +222,34 @@ struct EpiCG {
     rs[parity].store(rv, rhs, idx);
     return snorm2(rv);
   }
+  // same on the two spins of thread j of a pair (hop_pair_kernel); every lane of the warp calls
+  WL_D double half(int rhs, int parity, unsigned idx, int j, bool act, cplx<typename SF::real> (&acc)[2][3]) const {
+    using T = typename SF::real;
+    cplx<T> xv[2][3], rv[2][3];
+    double n = 0.0;
+    if (act) {
+      const double den = pAp[rhs];
+      const T al = (den > 0.0) ? T(r2[rhs] / den) : T(0);
+      const T aa = T(a[rhs]), bb = T(b[rhs]);
+      cplx<T> yv[2][3], pv[2][3];
+      half_load(y[parity], rhs, idx, j, yv);
+      half_load(p[parity], rhs, idx, j, pv);
+      half_load(xs[parity], rhs, idx, j, xv);
+      half_load(rs[parity], rhs, idx, j, rv);
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const cplx<T> ap = aa * yv[s][c] + bb * acc[s][c];
+          xv[s][c] = xv[s][c] + al * pv[s][c];
+          rv[s][c] = rv[s][c] - al * ap;
+        }
+      n = hnorm2(rv);
+    }
+    half_store(xs[parity], rhs, idx, j, act, xv);
+    half_store(rs[parity], rhs, idx, j, act, rv);
+    return n;
+  }
   // same on packed FP32 pairs; the order keeps at most two packed spinors live
   WL_D double packed(int rhs, int parity, unsigned idx, float2 (&acc)[12]) const {
     const float al = float(alpha[rhs]);
@@ -320,6 +348,31 @@ struct EpiResid {
         o.v[s][c] = {(typename SFS::real)r.re, (typename SFS::real)r.im};
       }
     rs[parity].store(o, rhs, idx);
+    return n;
+  }
+  // same on the two spins of thread j of a pair (hop_pair_kernel); every lane of the warp calls
+  WL_D double half(int rhs, int parity, unsigned idx, int j, bool act, cplx<double> (&acc)[2][3]) const {
+    cplx<typename SFS::real> o[2][3];
+    double n = 0.0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) o[s][c] = {0, 0};
+    if (act) {
+      cplx<double> yv[2][3], bv[2][3];
+      half_load(y[parity], rhs, idx, j, yv);
+      half_load(bvec[parity], rhs, idx, j, bv);
+      const double aa = a[rhs], bb = b[rhs];
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const cplx<double> r = bv[s][c] - (aa * yv[s][c] + bb * acc[s][c]);
+          n += norm2(r);
+          o[s][c] = {(typename SFS::real)r.re, (typename SFS::real)r.im};
+        }
+    }
+    half_store(rs[parity], rhs, idx, j, act, o);
     return n;
   }
 };
