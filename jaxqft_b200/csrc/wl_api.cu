@@ -29,6 +29,7 @@
 #include "wl_hop_fast.cuh"
 #include "wl_site.cuh"
 #include "wl_hop_mma.cuh"
+#include "wl_persist.cuh"
 
 using namespace wl;
 
@@ -150,9 +151,9 @@ struct IField {
   long long rstride() const { return chunks_of(prec) * vh * npar; }  // site-major layout: chunks per rhs
 };
 
-template <int P>
-static SpinorField<P> sf(const IField& f, int par) {
-  SpinorField<P> s;
+template <int P, bool NC = true>
+static SpinorField<P, NC> sf(const IField& f, int par) {
+  SpinorField<P, NC> s;
   using Ptr = decltype(s.ptr);
   const long long ch = chunks_of(P), vh = f.vh, n = f.nrhs;
   if (!f.rhs_inner) {
@@ -174,10 +175,10 @@ static SpinorField<P> sf(const IField& f, int par) {
   return s;
 }
 // field pair indexed by parity; for single-parity fields both entries alias par 0
-template <int P>
-static void sf2(const IField& f, SpinorField<P> (&o)[2]) {
-  o[0] = sf<P>(f, 0);
-  o[1] = f.npar == 2 ? sf<P>(f, 1) : o[0];
+template <int P, bool NC>
+static void sf2(const IField& f, SpinorField<P, NC> (&o)[2]) {
+  o[0] = sf<P, NC>(f, 0);
+  o[1] = f.npar == 2 ? sf<P, NC>(f, 1) : o[0];
 }
 
 static wl_status alloc_field(wl_ctx* ctx, IField& f, int prec, int vh, int nrhs, int npar, bool rhs_inner = false) {
@@ -1212,6 +1213,11 @@ struct wl_engine {
   long long run_seen = 0;          // run iterations already counted into g_launches
   unsigned long long run_gauge_id = 0;
   bool run_failed = false;
+  // persistent iterations of the solve graph (wl_persist.cuh)
+  bool persist = false;
+  unsigned* psync = nullptr;       // device: barrier arrivals of the current launch
+  int* perr = nullptr;             // device: set when a barrier wait ran out
+  double* ppart = nullptr;         // device: [2][n][blocks] partial sums
   bool ru_links12 = false;         // FP64 true residual with 12-real links (links unitary to 1e-12)
 };
 
@@ -1570,6 +1576,125 @@ static void enqueue_iteration(wl_engine* E, cudaStream_t st, int part) {
   g_launches++;
   cg_decide_kernel<<<1, 128, 0, st>>>(Sc, n, E->use_cond ? 1 : 0, E->cond, E->use_cond ? E->ru_iters : nullptr,
                                       E->lanes_mode ? 1 : 0);
+}
+
+// ------------------------------------------------------------------ persistent iterations
+// wl_solve runs its iterations in cg_persist_kernel while a hop is at most this much work per SM; beyond that the
+// ordinary launches, with more resident warps and their own tuned shapes, are faster.  Measured (B200, whole solves to
+// 1e-12, ordinary -> persistent), in target sites of one hop (both parities for the full operator) or warp tiles a SM:
+//   FP32/FP16, 1-3 slots, by sites: 14 (8^4, even-odd) 3.9 -> 3.3 ms; 140 (12^3x24) 7.6 -> 6.4; 280 18.2 -> 12.3;
+//     443 (16^3x32) 11.0 -> 9.5; 886 33 -> 25; beyond: 1081 (20^3x40) 26.7 -> 31.4, 2242 (24^3x48) 51 -> 60
+//   FP64 pairs, by sites: 28 (8^4, full) 7.5 -> 6.4 ms; 280 23.4 -> 22.9, two slots 45.6 -> 41.8; beyond: 443 20.5 -> 34
+//   FP16 lanes, by tiles: 7 (8^4, 12 slots) 3.9 -> 3.1 ms; 14 10.0 -> 7.2; beyond: 18 11.1 -> 11.4, 35 22.1 -> 22.9
+//   FP32 lanes, by tiles: 7 4.4 -> 3.3 ms; 35 32.4 -> 28.5; 110 107 -> 92; 140 92 -> 84
+constexpr int kPersistSites = 900, kPersistSitesD = 300, kPersistTilesH = 16, kPersistTilesS = 150;
+
+static long long persist_items(const wl_engine* E) {
+  const long long vh = E->ctx->g.Vh;
+  if (!E->lanes_mode) return vh * E->npar;
+  const int R = E->ts.lanes, spw = 32 / R;
+  return (vh + spw - 1) / spw * ((E->n + R - 1) / R) * E->npar;
+}
+
+static bool persist_applies(const wl_engine* E) {
+  static const int mode = [] {  // WL_PERSIST=0: never, 2: whatever the size (comparisons)
+    const char* e = std::getenv("WL_PERSIST");
+    return e ? std::atoi(e) : 1;
+  }();
+  // a forced hop shape is forced for the ordinary launches
+  if (mode == 0 || E->n > kPersistMaxSlots || !fast_hop_enabled() || std::getenv("WL_FORCE_TUNE")) return false;
+  if (E->lanes_mode && (E->ts.lanes == 0 || E->ts.mma)) return false;
+  if (persist_items(E) > (1LL << 30)) return false;
+  const long long most = E->lanes_mode ? (E->sprec == P_HALF ? kPersistTilesH : kPersistTilesS)
+                                       : (E->sprec == P_DOUBLE ? kPersistSitesD : kPersistSites);
+  return mode == 2 || persist_items(E) <= most * E->ctx->sm_count;
+}
+
+template <int S, int KIND, int R, bool HC, bool HA, int T>
+static cudaError_t launch_persist(wl_engine* E, PersistArgs<S, typename SloppyLinks<S>::type>& A, cudaStream_t st) {
+  using LS = typename SloppyLinks<S>::type;
+  const auto kernel = cg_persist_kernel<S, LS, KIND, R, HC, HA, T>;
+  const size_t smem = persist_smem<KIND, R, T>();
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const long long items = persist_items(E);
+  const int sms = E->ctx->sm_count;
+  long long per = (items + sms - 1) / sms;
+  if (KIND != PK_LANES) per = (per + 31) / 32 * 32;  // whole warps of sites
+  A.per = (int)per;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((items + per - 1) / per));
+  cfg.blockDim = dim3(T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  g_launches++;
+  return cudaLaunchKernelEx(&cfg, kernel, A);
+}
+
+template <int S>
+static cudaError_t enqueue_persist(wl_engine* E, cudaStream_t st) {
+  PersistArgs<S, typename SloppyLinks<S>::type> A{};
+  A.g = E->ctx->g;
+  A.links = SloppyLinks<S>::get(E->gauge);
+  sf2<S>(E->p, A.p);
+  sf2<S>(E->t1, A.t1);
+  sf2<S>(E->y, A.y);
+  sf2<S>(E->rs, A.rs);
+  const bool eo = E->prm.op == WL_SOLVE_EO_NORMAL;
+  sf2<S>(E->t1, A.et.out);
+  A.et.b = E->neg_half;
+  sf2<S>(E->y, A.ey.out);
+  sf2<S>(E->p, A.ey.self);
+  A.ey.has_self = 1;
+  sf2<S>(E->y, A.ec.y);
+  sf2<S>(E->p, A.ec.p);
+  sf2<S>(E->xs, A.ec.xs);
+  sf2<S>(E->rs, A.ec.rs);
+  A.ey.a = A.ec.a = eo ? E->one : E->m0;
+  A.ey.b = A.ec.b = eo ? E->half_alpha : E->neg_half;
+  A.ec.r2 = E->alpha;
+  A.ec.pAp = E->one;
+  A.ec.alpha = E->alpha;
+  sf2<S>(E->rs, A.fu.rs);
+  sf2<S>(E->p, A.fu.p);
+  A.fu.beta = E->beta;
+  A.alpha = E->alpha;
+  A.beta = E->beta;
+  A.sc = scalars_of(E);
+  A.partials = E->ppart;
+  A.arrived = E->psync;
+  A.err = E->perr;
+  A.n = E->n;
+  A.eo = eo;
+  A.group = E->lanes_mode ? 1 : 0;
+  cudaError_t e = cudaMemsetAsync(E->psync, 0, sizeof(unsigned), st);
+  if (e != cudaSuccess) return e;
+  // Threads per block: 512 leave 128 registers, which hold the stencils without spills; the FP64 pair form is fastest
+  // with 384 (168 registers: 21.6 ms a solve at 12^3x24, 24.5 with 512, 27.6 with 256).  FP32 sites with 256 threads
+  // 12.7 ms, 512 10.1 ms, 768 11.5 ms a solve at 16^3x32 (one build each).
+  if constexpr (S == P_DOUBLE) {
+    return launch_persist<S, PK_PAIR, 16, false, false, 384>(E, A, st);
+  } else {
+    if (!E->lanes_mode) return launch_persist<S, PK_SITE, 16, false, false, 512>(E, A, st);
+    if constexpr (S == P_HALF) {
+      if (half_color_enabled()) {
+        if (E->ts.lanes == 16) {
+          if (half_acc_enabled()) return launch_persist<S, PK_LANES, 16, true, true, 512>(E, A, st);
+          return launch_persist<S, PK_LANES, 16, true, false, 512>(E, A, st);
+        }
+        if (E->ts.lanes == 8) return launch_persist<S, PK_LANES, 8, true, false, 512>(E, A, st);
+        return launch_persist<S, PK_LANES, 4, true, false, 512>(E, A, st);
+      }
+    }
+    if (E->ts.lanes == 16) return launch_persist<S, PK_LANES, 16, false, false, 512>(E, A, st);
+    if (E->ts.lanes == 8) return launch_persist<S, PK_LANES, 8, false, false, 512>(E, A, st);
+    return launch_persist<S, PK_LANES, 4, false, false, 512>(E, A, st);
+  }
 }
 
 template <int S>
@@ -1952,6 +2077,9 @@ extern "C" void wl_engine_destroy(wl_engine* E) {
   cudaFree(E->ru_iters);
   cudaFree(E->loop_count);
   cudaFree(E->run_state);
+  cudaFree(E->psync);
+  cudaFree(E->perr);
+  cudaFree(E->ppart);
   if (E->h_pinned) cudaFreeHost(E->h_pinned);
   if (E->poll_ev) cudaEventDestroy(E->poll_ev);
   if (st) cudaStreamDestroy(st);
@@ -2035,10 +2163,14 @@ extern "C" wl_status wl_engine_create(wl_ctx* ctx, wl_gauge* G, const wl_solve_p
   const size_t nblk = (size_t)g.Vh + 64;
   if (e == cudaSuccess) e = cudaMalloc(&E->partials, sizeof(double) * nblk * n);
   if (e == cudaSuccess) e = cudaMalloc(&E->counters, sizeof(unsigned) * (n + 1));
-  if (e == cudaSuccess) e = cudaMallocHost(&E->h_pinned, sizeof(int) * (3 * n + 2));
+  if (e == cudaSuccess) e = cudaMallocHost(&E->h_pinned, sizeof(int) * (3 * n + 4));
   if (e == cudaSuccess) e = cudaMalloc(&E->ru_iters, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&E->loop_count, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&E->run_state, 4 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&E->psync, sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc(&E->perr, sizeof(int));
+  if (e == cudaSuccess && n <= kPersistMaxSlots)
+    e = cudaMalloc(&E->ppart, sizeof(double) * 2 * n * ctx->sm_count);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->poll_ev, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     ctx->err = std::string("engine allocation: ") + cudaGetErrorString(e);
@@ -2050,6 +2182,7 @@ extern "C" wl_status wl_engine_create(wl_ctx* ctx, wl_gauge* G, const wl_solve_p
   cudaMemsetAsync(E->counters, 0, sizeof(unsigned) * (n + 1), st);
   cudaMemsetAsync(E->ru_iters, 0, sizeof(int), st);
   cudaMemsetAsync(E->run_state, 0, 4 * sizeof(int), st);
+  cudaMemsetAsync(E->perr, 0, sizeof(int), st);
   double* d = E->dbl;
   E->r2 = d + 0 * n; E->r2_new = d + 1 * n; E->pAp = d + 2 * n; E->r2_true = d + 3 * n;
   E->rmax2 = d + 4 * n; E->b2 = d + 5 * n; E->tol2 = d + 6 * n; E->beta = d + 7 * n;
@@ -2070,6 +2203,7 @@ extern "C" wl_status wl_engine_create(wl_ctx* ctx, wl_gauge* G, const wl_solve_p
   E->td.pair = 1;  // FP64 fields site-major: the two-threads-per-site stencil
   if (E->lanes_mode) E->td = pick_update_tune(E, st);
   E->tsite = Tune{1, 128, 1};
+  E->persist = persist_applies(E);
   e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     ctx->err = std::string("engine set-up: ") + cudaGetErrorString(e);
@@ -2205,6 +2339,35 @@ static cudaError_t capture_iteration(wl_engine* E, cudaStream_t st, cudaGraph_t 
   return e;
 }
 
+// One round of the persistent form: the iterations up to the next reliable update in one cooperative kernel, the
+// update of the slots it named, and the bookkeeping that drives the enclosing WHILE node.
+static cudaError_t enqueue_persist_round(wl_engine* E, cudaStream_t st, const SolveLoop* loop) {
+  cudaError_t e;
+  switch (E->sprec) {
+    case P_HALF: e = enqueue_persist<P_HALF>(E, st); break;
+    case P_SINGLE: e = enqueue_persist<P_SINGLE>(E, st); break;
+    default: e = enqueue_persist<P_DOUBLE>(E, st); break;
+  }
+  enqueue_part(E, st, 2);
+  E->capture_loop = loop;
+  enqueue_part(E, st, 3);
+  E->capture_loop = nullptr;
+  return e;
+}
+
+static cudaError_t capture_persist(wl_engine* E, cudaStream_t st, cudaGraph_t g, const SolveLoop* loop,
+                                   long long* kernels) {
+  const long long before = g_launches.load();
+  cudaError_t e = cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  e = enqueue_persist_round(E, st, loop);
+  cudaGraph_t out = nullptr;
+  const cudaError_t e2 = cudaStreamEndCapture(st, &out);
+  *kernels = g_launches.load() - before;
+  g_launches = before;  // captured, not launched
+  return e != cudaSuccess ? e : e2;
+}
+
 static wl_status build_graph(wl_engine* E, cudaStream_t st) {
   wl_ctx* ctx = E->ctx;
   cudaGraph_t graph = nullptr;
@@ -2255,7 +2418,7 @@ static wl_status build_loop_graph(wl_engine* E, cudaStream_t st, bool run_mode =
     for (int m : E->h_maxiter) cap = std::max(cap, m);
     SolveLoop L{E->n_active, E->loop_count, cap + 8, wh, nullptr, nullptr, nullptr};
     if (run_mode) L = SolveLoop{E->n_active, E->run_state + 2, 0, wh, E->run_state, E->run_state + 1, E->run_state + 3};
-    e = capture_iteration(E, st, body, &L, &nk);
+    e = E->persist && !run_mode ? capture_persist(E, st, body, &L, &nk) : capture_iteration(E, st, body, &L, &nk);
   }
   cudaGraphExec_t& exec = run_mode ? E->grun : E->gloop;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
@@ -2558,6 +2721,8 @@ extern "C" wl_status wl_engine_retire(wl_engine* E, int slot, void* x, wl_solve_
 // One launch of the engine's whole-solve graph (built on first use, rebuilt when the gauge or
 // the iteration limit changed); *ran is false when the graph is unavailable and the caller
 // drives the iterations from the host instead.
+static const char* const kPersistTimeout = "a bounded device wait of the persistent iteration ran out";
+
 static wl_status run_loop_graph(wl_engine* E, bool* ran) {
   *ran = false;
   if (E->loop_failed) return WL_OK;
@@ -2580,7 +2745,9 @@ static wl_status run_loop_graph(wl_engine* E, bool* ran) {
   WL_CUDA(ctx, cudaMemsetAsync(E->loop_count, 0, sizeof(int), st));
   WL_CUDA(ctx, cudaGraphLaunch(E->gloop, st));
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 2 + n, E->loop_count, sizeof(int), cudaMemcpyDeviceToHost, st));
+  WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 4 + n, E->perr, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaStreamSynchronize(st));
+  if (E->h_pinned[4 + n]) WL_FAIL(ctx, WL_ERR_TIMEOUT, kPersistTimeout);
   g_launches += (long long)E->h_pinned[2 + n] * E->loop_kernels;
   *ran = true;
   return WL_OK;
@@ -2640,10 +2807,24 @@ extern "C" wl_status wl_solve(wl_ctx* ctx, wl_gauge* G, const wl_solve_params* p
   bool looped = false;
   if (s == WL_OK && E->prm.use_graph) s = run_loop_graph(E, &looped);
   if (looped) s = wl_engine_poll(E, nullptr, &n_active);  // status, counters, wait errors
-  while (s == WL_OK && !looped) {
+  while (s == WL_OK && !looped) {  // host-driven: the same rounds or iterations without the loop graph
     s = wl_engine_poll(E, nullptr, &n_active);
     if (s != WL_OK || n_active == 0) break;
     if (done_iters > (long long)E->prm.maxiter + 2 * chunk) break;  // host-side guard
+    if (E->persist) {
+      const cudaError_t e = enqueue_persist_round(E, engine_stream(E), nullptr);
+      int err = 0;
+      if (e != cudaSuccess) {
+        E->persist = false;  // no cooperative launch here: step the iterations
+        cudaGetLastError();
+      } else if (cudaMemcpyAsync(&err, E->perr, sizeof(int), cudaMemcpyDeviceToHost, engine_stream(E)) != cudaSuccess ||
+                 cudaStreamSynchronize(engine_stream(E)) != cudaSuccess || err) {
+        ctx->err = kPersistTimeout;
+        s = WL_ERR_TIMEOUT;
+      }
+      done_iters += 1;
+      continue;
+    }
     s = wl_engine_step(E, chunk);
     done_iters += chunk;
   }
