@@ -796,7 +796,8 @@ static bool site_hop(wl_ctx* ctx, wl_gauge* G, const void* in, void* out, const 
   const bool w32 = (((uintptr_t)in | (uintptr_t)out | (uintptr_t)self) & 31) == 0;
   if (kind == 3 && parity < 0 && w32 && tile_hop_launch<DAG>(ctx, A)) return true;
   const int per = parity < 0 ? 16 : 32;  // compact sites per block (of both parities, or of one)
-  const dim3 grid((unsigned)((g.Vh + per - 1) / per), nrhs);
+  const unsigned blocks = (unsigned)((g.Vh + per - 1) / per), rows = std::min(blocks, 65535u);
+  const dim3 grid(nrhs, rows, (blocks + rows - 1) / rows);  // fields fastest, then sites (y, z)
   g_launches++;
   if (w32 && ref_sector_enabled()) ref_pair_kernel<DAG, 4, true><<<grid, kRefSiteBlock, 0, ctx->stream>>>(A);
   else if (w32) ref_pair_kernel<DAG, 4><<<grid, kRefSiteBlock, 0, ctx->stream>>>(A);

@@ -407,11 +407,12 @@ __global__ void __launch_bounds__(kRefSiteBlock, WL_REFPAIR_MINB) ref_pair_kerne
   const Geom& g = A.g;
   const int j = threadIdx.x & 1;
   const double sg = 1.0 - 2.0 * j;
-  const int rhs = blockIdx.y;
+  // the fields of a batch are neighbours in the grid: they read the same links, from L2 after the first
+  const int sites = (int)(blockIdx.z * gridDim.y + blockIdx.y);
+  const int rhs = blockIdx.x;
   // compact site of this pair: 16 per warp, the block's two warps on the two parities or on 32 sites of one
   const int parity = A.parity < 0 ? (int)(threadIdx.x >> 5) : A.parity;
-  const int i = A.parity < 0 ? (int)blockIdx.x * 16 + (int)((threadIdx.x & 31) >> 1)
-                             : (int)blockIdx.x * 32 + (int)(threadIdx.x >> 1);
+  const int i = A.parity < 0 ? sites * 16 + (int)((threadIdx.x & 31) >> 1) : sites * 32 + (int)(threadIdx.x >> 1);
   const bool act = i < g.Vh;
   Site s{};
   cplx<double> Ac[3], Xc[3], Yc[3];
