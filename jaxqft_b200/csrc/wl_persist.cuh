@@ -18,7 +18,8 @@
 // resident (cooperative launch, one block per SM).  Every wait has an iteration limit; a block whose wait runs out
 // sets *err, deactivates all slots and returns, so that the remaining waits run out too and the solve ends with an
 // error instead of hanging.
-// Measured (B200, whole solves to 1e-12): 12 point sources on 8^4 in FP16 3.99 -> 3.15 ms, one even-odd FP32 solve at
+// Measured (B200, whole solves to 1e-12): 12 point sources on 8^4 in FP16 3.62 -> 2.71 ms (2.93 with links staged
+// every sweep), one even-odd FP32 solve at
 // 16^3x32 10.9 -> 9.4 ms, an MD update there (full-lattice FP32 solve) 12.0 -> 9.7 ms.  What is left of an iteration
 // at 16^3x32 is four hops at the L2's rate, five barriers of about a microsecond and the FP64 updates.
 #pragma once
@@ -214,7 +215,7 @@ struct WarpLinks {
 
 template <bool DAG, int R, bool HC, bool HA, class A_, class SF, class EPI>
 WL_D void sweep_lanes(const A_& A, const SF (&src)[2], int parity0, int npar, const EPI& epi, PersistState& st,
-                      double* partials, WarpLinks<R>& L) {
+                      double* partials, WarpLinks<R>* links, bool staged) {
   constexpr int SPW = 32 / R;
   const Geom& g = A.g;
   const int lane = threadIdx.x & 31;
@@ -225,13 +226,16 @@ WL_D void sweep_lanes(const A_& A, const SF (&src)[2], int parity0, int npar, co
   for (int t = blockIdx.x * A.per + (threadIdx.x >> 5); t < end; t += blockDim.x >> 5) {  // uniform per warp
     const int second = t >= tiles1, parity = parity0 ^ second, tt = t - second * tiles1;
     const int sg = tt / groups, gr = tt - sg * groups, site0 = sg * SPW;
-    __syncwarp();
-    for (int j = lane; j < 8 * SPW; j += 32) {
-      const int sl = j >> 3, q = j & 7;
-      if (site0 + sl < g.Vh)
-        L.nb[sl][q] = stage_link<HC>(g, A.links, parity, site0 + sl, q >> 1, q & 1, L.link[sl].l[q]);
+    WarpLinks<R>& L = links[R >= 8 ? parity : 0];
+    if (!staged) {
+      __syncwarp();
+      for (int j = lane; j < 8 * SPW; j += 32) {
+        const int sl = j >> 3, q = j & 7;
+        if (site0 + sl < g.Vh)
+          L.nb[sl][q] = stage_link<HC>(g, A.links, parity, site0 + sl, q >> 1, q & 1, L.link[sl].l[q]);
+      }
+      __syncwarp();
     }
-    __syncwarp();
     const int sl = lane / R, c = site0 + sl, rhs = gr * R + (lane % R);
     double v = 0.0;
     if (c < g.Vh && rhs < A.n && st.active[rhs]) {
@@ -290,10 +294,15 @@ WL_D void sweep_update(const A_& A, int npar, PersistState& st, const SF&) {
   }
 }
 
+// Link slots per warp: one per target parity where two fit, so that a warp with a single tile of each parity (the
+// even-odd operator on a lattice of a few thousand sites) stages its links once per launch instead of four times an
+// iteration.
+constexpr int persist_slots(int R) { return R >= 8 ? 2 : 1; }
+
 // Dynamic shared memory of a block of T threads (PK_LANES: staged links)
 template <int KIND, int R, int T>
 constexpr size_t persist_smem() {
-  return KIND == PK_LANES ? (T / 32) * sizeof(WarpLinks<R>) : 0;
+  return KIND == PK_LANES ? (T / 32) * persist_slots(R) * sizeof(WarpLinks<R>) : 0;
 }
 
 template <int S, class LS, int KIND, int R, bool HC, bool HA, int T>
@@ -318,11 +327,14 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
     mine = st.active[tid] != 0;
   }
   if (!__syncthreads_or(mine)) return;  // the same in every block
+  const bool keep = KIND == PK_LANES && R >= 8 && A.eo && A.per <= T / 32;
+  bool staged = false;  // the links of both parities are in shared memory (from the second iteration on)
   const auto hop = [&](auto dag, const SF(&src)[2], int parity0, int np, const auto& epi, double* partials) {
     constexpr bool DAG = decltype(dag)::value;
     if constexpr (KIND == PK_LANES)
       sweep_lanes<DAG, R, HC, HA>(A, src, parity0, np, epi, st, partials,
-                                  reinterpret_cast<WarpLinks<R>*>(dyn)[threadIdx.x >> 5]);
+                                  reinterpret_cast<WarpLinks<R>*>(dyn) + (threadIdx.x >> 5) * persist_slots(R),
+                                  staged && keep);
     else if constexpr (KIND == PK_PAIR) sweep_pair<DAG>(A, src, parity0, np, epi, st, partials);
     else sweep_site<DAG>(A, src, parity0, np, epi, st, partials);
   };
@@ -330,7 +342,7 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
   const std::true_type dagger{};
   unsigned target = 0;
   bool ok = true;
-  while (true) {
+  for (;; staged = true) {
     // ---- y = M p (or D p), pAp = |y|^2
     if (A.eo) {
       hop(plain, A.p, 1, 1, A.et, nullptr);
