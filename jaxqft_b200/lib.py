@@ -219,6 +219,8 @@ class WilsonContext:
             raise ValueError("every lattice extent must be even and >= 2 (even/odd layout)")
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
         self.volume = int(np.prod(self.lattice_shape))
+        self._torch, self._index, self._field = torch, int(self.device.index or 0), 12 * self.volume
+        self._wl_apply = self.lib.wl_apply
         g = WLGeometry()
         for mu in range(4):
             g.dims[mu] = self.lattice_shape[mu]
@@ -249,19 +251,24 @@ class WilsonContext:
     # ------------------------------------------------------------ operators
     def apply(self, op: str, gauge: Gauge, mass: float, psi, normalized: bool = False, out=None):
         """out = op(psi) for psi of shape (nrhs, Lx, Ly, Lz, Lt, 4, 3) or (Lx..Lt, 4, 3)."""
-        import torch
-
-        psi = _c128(psi, self.device)
-        nrhs = psi.numel() // (12 * self.volume)
-        if nrhs * 12 * self.volume != psi.numel():
-            raise ValueError(f"field of {psi.numel()} elements does not match lattice {self.lattice_shape}")
+        # on a small lattice this call is bound by the host: a field that needs no conversion takes none of the checks
+        # of _c128 twice
+        torch = self._torch
+        if not (type(psi) is torch.Tensor and psi.dtype is torch.complex128 and psi.get_device() == self._index
+                and psi.is_contiguous()):
+            psi = _c128(psi, self.device)
+        n = psi.numel()
+        nrhs = n // self._field
+        if nrhs * self._field != n:
+            raise ValueError(f"field of {n} elements does not match lattice {self.lattice_shape}")
         if out is None:
             out = torch.empty_like(psi)
         if nrhs == 0:  # an empty batch maps to an empty result, as the reference's vmapped operators do
             return out
-        flags = FLAG_NORMALIZED if normalized else 0
-        self._check(self.lib.wl_apply(self.handle, gauge.handle, OPS[op], float(mass), flags, _ptr(psi), _ptr(out),
-                                      nrhs))
+        rc = self._wl_apply(self.handle, gauge.handle, OPS[op], float(mass), FLAG_NORMALIZED if normalized else 0,
+                            psi.data_ptr(), out.data_ptr(), nrhs)
+        if rc:
+            self._check(rc)
         return out
 
     def pf_force(self, gauge: Gauge, X, Y, coef: float = 1.0, F=None):
