@@ -1614,7 +1614,8 @@ static bool persist_applies(const wl_engine* E) {
 template <int S, int KIND, int R, bool HC, bool HA, int T>
 static cudaError_t launch_persist(wl_engine* E, PersistArgs<S, typename SloppyLinks<S>::type>& A, cudaStream_t st) {
   using LS = typename SloppyLinks<S>::type;
-  const auto kernel = cg_persist_kernel<S, LS, KIND, R, HC, HA, T>;
+  const auto kernel = E->prm.op == WL_SOLVE_EO_NORMAL ? cg_persist_kernel<S, LS, KIND, R, HC, HA, T, true>
+                                                      : cg_persist_kernel<S, LS, KIND, R, HC, HA, T, false>;
   const size_t smem = persist_smem<KIND, R, T>();
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -1671,7 +1672,6 @@ static cudaError_t enqueue_persist(wl_engine* E, cudaStream_t st) {
   A.arrived = E->psync;
   A.err = E->perr;
   A.n = E->n;
-  A.eo = eo;
   A.group = E->lanes_mode ? 1 : 0;
   cudaError_t e = cudaMemsetAsync(E->psync, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;

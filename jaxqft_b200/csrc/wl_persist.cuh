@@ -18,10 +18,11 @@
 // resident (cooperative launch, one block per SM).  Every wait has an iteration limit; a block whose wait runs out
 // sets *err, deactivates all slots and returns, so that the remaining waits run out too and the solve ends with an
 // error instead of hanging.
-// Measured (B200, whole solves to 1e-12): 12 point sources on 8^4 in FP16 3.62 -> 2.71 ms (2.93 with links staged
-// every sweep), one even-odd FP32 solve at
-// 16^3x32 10.9 -> 9.4 ms, an MD update there (full-lattice FP32 solve) 12.0 -> 9.7 ms.  What is left of an iteration
-// at 16^3x32 is four hops at the L2's rate, five barriers of about a microsecond and the FP64 updates.
+// Measured (B200, whole solves to 1e-12, ordinary launches -> this kernel): 12 point sources on 8^4 in FP16 3.97 ->
+// 2.66 ms (links staged every sweep 2.93), one even-odd FP32 solve at 16^3x32 10.8 -> 9.1 ms, plain FP64 CG at
+// 12^3x24 23.3 -> 20.4 ms, an MD update at 16^3x32 (full-lattice FP32 solve) 11.9 -> 8.6 ms.  What is left of an
+// iteration at 16^3x32 is four hops at the L2's rate and latency, five barriers of 1.5-2.6 us and the FP64 updates.
+// Measured and not kept: the loads of two (FP32) or four (FP16) hops issued together (spills; 9.8 against 9.5 ms).
 #pragma once
 #include "wl_site.cuh"
 
@@ -48,7 +49,7 @@ struct PersistArgs {
   unsigned* arrived; // barrier arrivals of this launch, zero before it
   int* err;
   int n;             // slots, <= kPersistMaxSlots
-  int eo, group;
+  int group;
   int per;           // sites (PK_SITE, PK_PAIR; a multiple of 32) or warp tiles (PK_LANES) per block
 };
 
@@ -163,7 +164,7 @@ WL_D void sweep_site(const A_& A, const SF (&src)[2], int parity0, int npar, con
     const int i = first + (int)(threadIdx.x & 31);
     double v = 0.0;
     if (i < end) {
-      const int second = i >= g.Vh, parity = parity0 ^ second, c = i - second * g.Vh;
+      const int second = npar == 2 && i >= g.Vh, parity = parity0 ^ second, c = i - second * g.Vh;
       const Site s = site_from_compact(g, parity, c);
       const bool act[1] = {true};
       const auto links = opaque_links(A.links);
@@ -195,7 +196,7 @@ WL_D void sweep_pair(const A_& A, const SF (&src)[2], int parity0, int npar, con
   for_items<16>(A, npar, st, [&](int rhs, int first, int end) {
     const int i = first + (int)((threadIdx.x & 31) >> 1);
     const bool act = i < end;
-    const int second = i >= g.Vh, parity = parity0 ^ second, c = i - second * g.Vh;
+    const int second = npar == 2 && i >= g.Vh, parity = parity0 ^ second, c = i - second * g.Vh;
     Site s{};
     if (act) s = site_from_compact(g, parity, c);
     cplx<T> o[2][3];
@@ -224,7 +225,7 @@ WL_D void sweep_lanes(const A_& A, const SF (&src)[2], int parity0, int npar, co
   if (EPI::kReduce) sweep_begin(st);
 #pragma unroll 1
   for (int t = blockIdx.x * A.per + (threadIdx.x >> 5); t < end; t += blockDim.x >> 5) {  // uniform per warp
-    const int second = t >= tiles1, parity = parity0 ^ second, tt = t - second * tiles1;
+    const int second = npar == 2 && t >= tiles1, parity = parity0 ^ second, tt = t - second * tiles1;
     const int sg = tt / groups, gr = tt - sg * groups, site0 = sg * SPW;
     WarpLinks<R>& L = links[R >= 8 ? parity : 0];
     if (!staged) {
@@ -263,7 +264,7 @@ WL_D void sweep_update(const A_& A, int npar, PersistState& st, const SF&) {
     const int lane = threadIdx.x & 31, groups = (A.n + R - 1) / R, tiles1 = ((g.Vh + SPW - 1) / SPW) * groups;
     const int end = min((int)(blockIdx.x + 1) * A.per, npar * tiles1);
     for (int t = blockIdx.x * A.per + (threadIdx.x >> 5); t < end; t += blockDim.x >> 5) {
-      const int parity = t >= tiles1, tt = t - parity * tiles1, sg = tt / groups;
+      const int parity = npar == 2 && t >= tiles1, tt = t - parity * tiles1, sg = tt / groups;
       const int c = sg * SPW + lane / R, rhs = (tt - sg * groups) * R + lane % R;
       if (c < g.Vh && rhs < A.n && st.active[rhs]) A.fu(rhs, parity, c);
     }
@@ -274,7 +275,7 @@ WL_D void sweep_update(const A_& A, int npar, PersistState& st, const SF&) {
       const int i = first + (int)((threadIdx.x & 31) >> 1);
       if (i >= end) return;
       const T be = T(st.beta[rhs]);
-      const int parity = i >= g.Vh, c = i - parity * g.Vh;
+      const int parity = npar == 2 && i >= g.Vh, c = i - parity * g.Vh;
       cplx<T> r[2][3], q[2][3];
       half_load(A.rs[parity], rhs, c, j, r);
       half_load(A.p[parity], rhs, c, j, q);
@@ -288,7 +289,7 @@ WL_D void sweep_update(const A_& A, int npar, PersistState& st, const SF&) {
     for_items<32>(A, npar, st, [&](int rhs, int first, int end) {
       const int i = first + (int)(threadIdx.x & 31);
       if (i >= end) return;
-      const int parity = i >= g.Vh;
+      const int parity = npar == 2 && i >= g.Vh;
       A.fu(rhs, parity, i - parity * g.Vh);
     });
   }
@@ -305,13 +306,15 @@ constexpr size_t persist_smem() {
   return KIND == PK_LANES ? (T / 32) * persist_slots(R) * sizeof(WarpLinks<R>) : 0;
 }
 
-template <int S, class LS, int KIND, int R, bool HC, bool HA, int T>
+// EO (the even-odd operator, four hops) and the full operator (two) are separate instantiations: sharing one function
+// their sweeps were merged and spilled (FP64 600 bytes a thread against 120; solves 5-15 % slower).
+template <int S, class LS, int KIND, int R, bool HC, bool HA, int T, bool EO>
 __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant__ PersistArgs<S, LS> A) {
   using SF = SpinorField<S, false>;
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ PersistState st;
   const int tid = threadIdx.x;
-  const int npar = A.eo ? 1 : 2;
+  constexpr int npar = EO ? 1 : 2;
   double* part0 = A.partials;
   double* part1 = A.partials + (size_t)A.n * gridDim.x;
   bool mine = false;
@@ -327,7 +330,7 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
     mine = st.active[tid] != 0;
   }
   if (!__syncthreads_or(mine)) return;  // the same in every block
-  const bool keep = KIND == PK_LANES && R >= 8 && A.eo && A.per <= T / 32;
+  const bool keep = KIND == PK_LANES && R >= 8 && EO && A.per <= T / 32;
   bool staged = false;  // the links of both parities are in shared memory (from the second iteration on)
   const auto hop = [&](auto dag, const SF(&src)[2], int parity0, int np, const auto& epi, double* partials) {
     constexpr bool DAG = decltype(dag)::value;
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
   bool ok = true;
   for (;; staged = true) {
     // ---- y = M p (or D p), pAp = |y|^2
-    if (A.eo) {
+    if constexpr (EO) {
       hop(plain, A.p, 1, 1, A.et, nullptr);
       if (!(ok = grid_barrier(A.arrived, target, st))) break;
       hop(plain, A.t1, 0, 1, A.ey, part0);
@@ -356,7 +359,7 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
     if (tid < A.n && st.active[tid]) A.alpha[tid] = st.pap[tid] > 0.0 ? st.r2[tid] / st.pap[tid] : 0.0;
     __syncthreads();
     // ---- x_s += alpha p, r_s -= alpha M^dag y, r2n = |r_s|^2
-    if (A.eo) {
+    if constexpr (EO) {
       hop(dagger, A.y, 1, 1, A.et, nullptr);
       if (!(ok = grid_barrier(A.arrived, target, st))) break;
       hop(dagger, A.t1, 0, 1, A.ec, part1);
