@@ -29,6 +29,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-shared",
     "--expt-relaxed-constexpr",
     "-Xptxas", "-O3",
+    "--split-compile=0",  # optimise and assemble the kernels of the one source file on all cores
 ]
 
 

@@ -1582,13 +1582,16 @@ static void enqueue_iteration(wl_engine* E, cudaStream_t st, int part) {
 // ------------------------------------------------------------------ persistent iterations
 // wl_solve runs its iterations in cg_persist_kernel while a hop is at most this much work per SM; beyond that the
 // ordinary launches, with more resident warps and their own tuned shapes, are faster.  Measured (B200, whole solves to
-// 1e-12, ordinary -> persistent), in target sites of one hop (both parities for the full operator) or warp tiles a SM:
-//   FP32/FP16, 1-3 slots, by sites: 14 (8^4, even-odd) 3.9 -> 3.3 ms; 140 (12^3x24) 7.6 -> 6.4; 280 18.2 -> 12.3;
-//     443 (16^3x32) 11.0 -> 9.5; 886 33 -> 25; beyond: 1081 (20^3x40) 26.7 -> 31.4, 2242 (24^3x48) 51 -> 60
-//   FP64 pairs, by sites: 28 (8^4, full) 7.5 -> 6.4 ms; 280 23.4 -> 22.9, two slots 45.6 -> 41.8; beyond: 443 20.5 -> 34
-//   FP16 lanes, by tiles: 7 (8^4, 12 slots) 3.9 -> 3.1 ms; 14 10.0 -> 7.2; beyond: 18 11.1 -> 11.4, 35 22.1 -> 22.9
-//   FP32 lanes, by tiles: 7 4.4 -> 3.3 ms; 35 32.4 -> 28.5; 110 107 -> 92; 140 92 -> 84
-constexpr int kPersistSites = 900, kPersistSitesD = 300, kPersistTilesH = 16, kPersistTilesS = 150;
+// 1e-12, ordinary -> persistent ms), in target sites of one hop (both parities for the full operator) or warp tiles a SM:
+//   FP32 sites (1-3 slots): 14 (8^4, even-odd) 3.8 -> 3.1; 140 (12^3x24) 7.5 -> 5.9; 280 17.5 -> 10.9; 443 (16^3x32)
+//     10.8 -> 9.1; 886 31.5 -> 22.6, two slots 62.8 -> 45.1; beyond: 1081 (20^3x40) 27.3 -> 26.7, 2242 (24^3x48)
+//     51 -> 54.  FP16 sites: 443 12.3 -> 10.4; beyond: 1081 23.4 -> 23.9, 2242 48 -> 54
+//   FP64 pairs, by sites: 28 (8^4, full) 7.3 -> 5.6; 280 23.4 -> 20.3, two slots 46.2 -> 35.9; beyond: 443 20.7 -> 30.2
+//     Two and three slots only while each of the block's 12 warps gets one item (190 sites x slots a SM): beyond, a
+//     second, part-empty sweep made them 0.81-1.15 of the ordinary time (74 x 3: 5.1 -> 6.4; 91 x 3: 12.5 -> 10.9).
+//   FP16 lanes, by tiles: 7 (8^4, 12 slots) 4.0 -> 2.7; 18 (12^3x24) 11.0 -> 10.4; 35 22.0 -> 21.0; 55 28.6 -> 26.0
+//   FP32 lanes, by tiles: 7 4.3 -> 2.8; 35 32.3 -> 26.7; 110 108 -> 90; 140 92 -> 82
+constexpr int kPersistSites = 900, kPersistSitesD = 300, kPersistSlotSitesD = 190, kPersistTilesH = 60, kPersistTilesS = 150;
 
 static long long persist_items(const wl_engine* E) {
   const long long vh = E->ctx->g.Vh;
@@ -1605,10 +1608,15 @@ static bool persist_applies(const wl_engine* E) {
   // a forced hop shape is forced for the ordinary launches
   if (mode == 0 || E->n > kPersistMaxSlots || !fast_hop_enabled() || std::getenv("WL_FORCE_TUNE")) return false;
   if (E->lanes_mode && (E->ts.lanes == 0 || E->ts.mma)) return false;
+  if (E->lanes_mode && E->sprec == P_HALF && !(half_color_enabled() && half_acc_enabled())) return false;
   if (persist_items(E) > (1LL << 30)) return false;
   const long long most = E->lanes_mode ? (E->sprec == P_HALF ? kPersistTilesH : kPersistTilesS)
                                        : (E->sprec == P_DOUBLE ? kPersistSitesD : kPersistSites);
-  return mode == 2 || persist_items(E) <= most * E->ctx->sm_count;
+  if (mode == 2) return true;
+  if (!E->lanes_mode && E->sprec == P_DOUBLE && E->n > 1 &&
+      persist_items(E) * E->n > (long long)kPersistSlotSitesD * E->ctx->sm_count)
+    return false;
+  return persist_items(E) <= most * E->ctx->sm_count;
 }
 
 template <int S, int KIND, int R, bool HC, bool HA, int T>
@@ -1622,7 +1630,10 @@ static cudaError_t launch_persist(wl_engine* E, PersistArgs<S, typename SloppyLi
   const long long items = persist_items(E);
   const int sms = E->ctx->sm_count;
   long long per = (items + sms - 1) / sms;
-  if (KIND != PK_LANES) per = (per + 31) / 32 * 32;  // whole warps of sites
+  if (KIND != PK_LANES) {  // whole warps of sites
+    const int w = KIND == PK_PAIR ? 16 : 32;
+    per = (per + w - 1) / w * w;
+  }
   A.per = (int)per;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)((items + per - 1) / per));
@@ -1682,19 +1693,10 @@ static cudaError_t enqueue_persist(wl_engine* E, cudaStream_t st) {
     return launch_persist<S, PK_PAIR, 16, false, false, 384>(E, A, st);
   } else {
     if (!E->lanes_mode) return launch_persist<S, PK_SITE, 16, false, false, 512>(E, A, st);
-    if constexpr (S == P_HALF) {
-      if (half_color_enabled()) {
-        if (E->ts.lanes == 16) {
-          if (half_acc_enabled()) return launch_persist<S, PK_LANES, 16, true, true, 512>(E, A, st);
-          return launch_persist<S, PK_LANES, 16, true, false, 512>(E, A, st);
-        }
-        if (E->ts.lanes == 8) return launch_persist<S, PK_LANES, 8, true, false, 512>(E, A, st);
-        return launch_persist<S, PK_LANES, 4, true, false, 512>(E, A, st);
-      }
-    }
-    if (E->ts.lanes == 16) return launch_persist<S, PK_LANES, 16, false, false, 512>(E, A, st);
-    if (E->ts.lanes == 8) return launch_persist<S, PK_LANES, 8, false, false, 512>(E, A, st);
-    return launch_persist<S, PK_LANES, 4, false, false, 512>(E, A, st);
+    constexpr bool H = S == P_HALF;  // FP16: packed colour multiply, and with 16 lanes FP16 accumulation
+    if (E->ts.lanes == 16) return launch_persist<S, PK_LANES, 16, H, H, 512>(E, A, st);
+    if (E->ts.lanes == 8) return launch_persist<S, PK_LANES, 8, H, false, 512>(E, A, st);
+    return launch_persist<S, PK_LANES, 4, H, false, 512>(E, A, st);
   }
 }
 

@@ -50,7 +50,7 @@ struct PersistArgs {
   int* err;
   int n;             // slots, <= kPersistMaxSlots
   int group;
-  int per;           // sites (PK_SITE, PK_PAIR; a multiple of 32) or warp tiles (PK_LANES) per block
+  int per;           // sites (PK_SITE, PK_PAIR: whole warps) or warp tiles (PK_LANES) per block
 };
 
 struct PersistState {
