@@ -2724,6 +2724,13 @@ extern "C" wl_status wl_engine_retire(wl_engine* E, int slot, void* x, wl_solve_
 // One launch of the engine's whole-solve graph (built on first use, rebuilt when the gauge or
 // the iteration limit changed); *ran is false when the graph is unavailable and the caller
 // drives the iterations from the host instead.
+// Persistent solves of one device take turns: two of them, each with a block per SM, could otherwise hold half of the
+// SMs each and wait for the other's blocks.  Held from the launch to the synchronisation that ends it.
+static std::mutex g_persist_mu[64];
+static std::unique_lock<std::mutex> persist_turn(const wl_engine* E) {
+  return E->persist ? std::unique_lock<std::mutex>(g_persist_mu[E->ctx->device & 63]) : std::unique_lock<std::mutex>();
+}
+
 static const char* const kPersistTimeout = "a bounded device wait of the persistent iteration ran out";
 
 static wl_status run_loop_graph(wl_engine* E, bool* ran) {
@@ -2746,6 +2753,7 @@ static wl_status run_loop_graph(wl_engine* E, bool* ran) {
   }
   const int n = E->n;
   WL_CUDA(ctx, cudaMemsetAsync(E->loop_count, 0, sizeof(int), st));
+  const auto turn = persist_turn(E);
   WL_CUDA(ctx, cudaGraphLaunch(E->gloop, st));
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 2 + n, E->loop_count, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 4 + n, E->perr, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2815,6 +2823,7 @@ extern "C" wl_status wl_solve(wl_ctx* ctx, wl_gauge* G, const wl_solve_params* p
     if (s != WL_OK || n_active == 0) break;
     if (done_iters > (long long)E->prm.maxiter + 2 * chunk) break;  // host-side guard
     if (E->persist) {
+      const auto turn = persist_turn(E);
       const cudaError_t e = enqueue_persist_round(E, engine_stream(E), nullptr);
       int err = 0;
       if (e != cudaSuccess) {
