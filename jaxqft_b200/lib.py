@@ -271,12 +271,18 @@ class WilsonContext:
             self._check(rc)
         return out
 
+    def _one_field(self, x, name):
+        """One spinor field of the whole lattice as the force kernels read it: complex128, contiguous, on this device."""
+        x = _c128(x, self.device)
+        if x.numel() != self._field:
+            raise ValueError(f"{name} of {x.numel()} elements is not one field on lattice {self.lattice_shape}")
+        return x
+
     def pf_force(self, gauge: Gauge, X, Y, coef: float = 1.0, F=None):
         """F (+)= coef * pseudofermion_force_from_solution(U, X, Y) for one configuration."""
         import torch
 
-        X = _c128(X, self.device)
-        Y = _c128(Y, self.device)
+        X, Y = self._one_field(X, "X"), self._one_field(Y, "Y")
         acc = F is not None
         if F is None:
             F = torch.empty((4, *self.lattice_shape, 3, 3), dtype=torch.complex128, device=self.device)
@@ -286,9 +292,10 @@ class WilsonContext:
 
     def _force_into(self, gauge: Gauge, X, Y, F, eo_coef: Optional[float] = None):
         """F = the force of X, Y (pf_force), or with eo_coef the even-odd force of X_e, Y_e times
-        eo_coef; complex128 fields of one configuration on this device, F overwritten."""
+        eo_coef; fields of one configuration, F (complex128, contiguous, on this device) overwritten."""
         import torch
 
+        X, Y = self._one_field(X, "X"), self._one_field(Y, "Y")
         if eo_coef is None:
             self._check(self.lib.wl_pf_force(self.handle, gauge.handle, _ptr(X), _ptr(Y), 1.0, 0, _ptr(F)))
             return
