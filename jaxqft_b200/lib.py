@@ -236,7 +236,21 @@ class WilsonContext:
         self.set_stream(torch.cuda.current_stream(self.device))
 
     def set_stream(self, stream):
-        self._check(self.lib.wl_ctx_set_stream(self.handle, ctypes.c_void_p(int(stream.cuda_stream))))
+        self._stream = int(stream.cuda_stream)
+        self._check(self.lib.wl_ctx_set_stream(self.handle, ctypes.c_void_p(self._stream)))
+
+    def _scratch(self, *shape):
+        """Uninitialised complex128 scratch that may be dropped while kernels of this context still use it: a block of
+        the context's stream, which the caching allocator gives only to work queued behind them.  (A block of another
+        current stream would be free for that stream's next tensor as soon as it is dropped.)"""
+        torch = self._torch
+        make = lambda: torch.empty(shape, dtype=torch.complex128, device=self.device)  # noqa: E731
+        if torch.cuda.current_stream(self.device).cuda_stream == self._stream:
+            return make()
+        own = (torch.cuda.ExternalStream(self._stream, device=self.device) if self._stream
+               else torch.cuda.default_stream(self.device))
+        with torch.cuda.stream(own):
+            return make()
 
     def _check(self, rc: int):
         if rc != WL_OK:
@@ -293,13 +307,11 @@ class WilsonContext:
     def _force_into(self, gauge: Gauge, X, Y, F, eo_coef: Optional[float] = None):
         """F = the force of X, Y (pf_force), or with eo_coef the even-odd force of X_e, Y_e times
         eo_coef; fields of one configuration, F (complex128, contiguous, on this device) overwritten."""
-        import torch
-
         X, Y = self._one_field(X, "X"), self._one_field(Y, "Y")
         if eo_coef is None:
             self._check(self.lib.wl_pf_force(self.handle, gauge.handle, _ptr(X), _ptr(Y), 1.0, 0, _ptr(F)))
             return
-        scratch = torch.empty((2, *self.lattice_shape, 4, 3), dtype=torch.complex128, device=self.device)
+        scratch = self._scratch(2, *self.lattice_shape, 4, 3)
         self._check(self.lib.wl_pf_force_eo(self.handle, gauge.handle, _ptr(X), _ptr(Y), float(eo_coef),
                                             _ptr(scratch), _ptr(F)))
 
@@ -318,7 +330,7 @@ class WilsonContext:
         U, B = self._links(U, "U")
         if out is None:
             out = torch.empty_like(U)
-        scratch = torch.empty_like(U)  # element-major copy of the links, from the caching allocator
+        scratch = self._scratch(*U.shape)  # element-major copy of the links
         self._check(self.lib.wl_gauge_force_ws(self.handle, _ptr(U), B, float(beta), _ptr(scratch), _ptr(out)))
         return out
 
