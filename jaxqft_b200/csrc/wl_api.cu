@@ -1600,11 +1600,17 @@ static long long persist_items(const wl_engine* E) {
   return (vh + spw - 1) / spw * ((E->n + R - 1) / R) * E->npar;
 }
 
-static bool persist_applies(const wl_engine* E) {
-  static const int mode = [] {  // WL_PERSIST=0: never, 2: whatever the size (comparisons)
+// WL_PERSIST=0: never, 2: whatever the size (comparisons), 3: every launch refused (the fallback)
+static int persist_mode() {
+  static const int mode = [] {
     const char* e = std::getenv("WL_PERSIST");
     return e ? std::atoi(e) : 1;
   }();
+  return mode;
+}
+
+static bool persist_applies(const wl_engine* E) {
+  const int mode = persist_mode();
   // a forced hop shape is forced for the ordinary launches
   if (mode == 0 || E->n > kPersistMaxSlots || !fast_hop_enabled() || std::getenv("WL_FORCE_TUNE")) return false;
   if (E->lanes_mode && (E->ts.lanes == 0 || E->ts.mma)) return false;
@@ -1624,6 +1630,7 @@ static cudaError_t launch_persist(wl_engine* E, PersistArgs<S, typename SloppyLi
   using LS = typename SloppyLinks<S>::type;
   const auto kernel = E->prm.op == WL_SOLVE_EO_NORMAL ? cg_persist_kernel<S, LS, KIND, R, HC, HA, T, true>
                                                       : cg_persist_kernel<S, LS, KIND, R, HC, HA, T, false>;
+  if (persist_mode() == 3) return cudaErrorCooperativeLaunchTooLarge;
   const size_t smem = persist_smem<KIND, R, T>();
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -2343,7 +2350,8 @@ static cudaError_t capture_iteration(wl_engine* E, cudaStream_t st, cudaGraph_t 
 }
 
 // One round of the persistent form: the iterations up to the next reliable update in one cooperative kernel, the
-// update of the slots it named, and the bookkeeping that drives the enclosing WHILE node.
+// update of the slots it named, and the bookkeeping that drives the enclosing WHILE node.  When the cooperative launch
+// is refused nothing else is enqueued either: the solver state stays as it was, and the caller steps on from it.
 static cudaError_t enqueue_persist_round(wl_engine* E, cudaStream_t st, const SolveLoop* loop) {
   cudaError_t e;
   switch (E->sprec) {
@@ -2351,6 +2359,7 @@ static cudaError_t enqueue_persist_round(wl_engine* E, cudaStream_t st, const So
     case P_SINGLE: e = enqueue_persist<P_SINGLE>(E, st); break;
     default: e = enqueue_persist<P_DOUBLE>(E, st); break;
   }
+  if (e != cudaSuccess) return e;
   enqueue_part(E, st, 2);
   E->capture_loop = loop;
   enqueue_part(E, st, 3);
@@ -2744,17 +2753,27 @@ static wl_status run_loop_graph(wl_engine* E, bool* ran) {
     cudaGraphExecDestroy(E->gloop);
     E->gloop = nullptr;
   }
-  if (!E->gloop) {
-    if (build_loop_graph(E, st) != WL_OK) {
-      ctx->err.clear();
-      return WL_OK;
-    }
-    E->loop_gauge_id = E->gauge->id;
-  }
   const int n = E->n;
   WL_CUDA(ctx, cudaMemsetAsync(E->loop_count, 0, sizeof(int), st));
   const auto turn = persist_turn(E);
-  WL_CUDA(ctx, cudaGraphLaunch(E->gloop, st));
+  for (;;) {
+    cudaError_t e = cudaErrorNotSupported;
+    if (E->gloop || build_loop_graph(E, st) == WL_OK) {
+      E->loop_gauge_id = E->gauge->id;
+      e = cudaGraphLaunch(E->gloop, st);
+    }
+    if (e == cudaSuccess) break;
+    if (E->persist) {  // no cooperative kernel in a loop body here, and nothing ran: loop over the ordinary iteration
+      cudaGetLastError();
+      if (E->gloop) cudaGraphExecDestroy(E->gloop);
+      E->gloop = nullptr;
+      E->persist = E->loop_failed = false;
+      continue;
+    }
+    if (E->gloop) WL_CUDA(ctx, e);
+    ctx->err.clear();
+    return WL_OK;
+  }
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 2 + n, E->loop_count, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 4 + n, E->perr, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaStreamSynchronize(st));
