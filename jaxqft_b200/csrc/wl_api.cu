@@ -1163,6 +1163,19 @@ std::map<TuneKey, Tune> g_tune_cache;
 
 }  // namespace
 
+// A solve as one graph (a WHILE node over the iteration or over the persistent round), launched once per wl_solve
+struct SolveLoopGraph {
+  cudaGraphExec_t exec = nullptr;
+  long long kernels = 0;           // unconditional kernels per pass of the loop
+  int cap = 0;                     // maxiter it was built for
+  unsigned long long gauge_id = 0;
+  bool failed = false;             // it could not be built or launched
+  void release() {
+    if (exec) cudaGraphExecDestroy(exec);
+    exec = nullptr;
+  }
+};
+
 struct wl_engine {
   wl_ctx* ctx = nullptr;
   wl_gauge* gauge = nullptr;
@@ -1199,13 +1212,8 @@ struct wl_engine {
   cudaGraphConditionalHandle cond = 0;
   int* ru_iters = nullptr;         // device: iterations whose conditional body ran
   long long ru_iters_seen = 0;
-  // the solve as one graph (WHILE node over the iteration), launched once per wl_solve
-  cudaGraphExec_t gloop = nullptr;
-  int* loop_count = nullptr;       // device: iterations run by the loop graph's current launch
-  long long loop_kernels = 0;      // unconditional kernels per loop iteration
-  int loop_cap = 0;                // maxiter the loop graph was built for
-  unsigned long long loop_gauge_id = 0;
-  bool loop_failed = false;        // the loop graph could not be built: host-driven loop
+  SolveLoopGraph loop, ploop;      // over the ordinary iteration, over the persistent round
+  int* loop_count = nullptr;       // device: passes run by the loop graph's current launch
   const SolveLoop* capture_loop = nullptr;  // set while part 3 of a loop body is captured
   // engine run (wl_engine_run): WHILE node that stops when a slot finishes or at a per-launch cap
   cudaGraphExec_t grun = nullptr;
@@ -1214,7 +1222,7 @@ struct wl_engine {
   long long run_seen = 0;          // run iterations already counted into g_launches
   unsigned long long run_gauge_id = 0;
   bool run_failed = false;
-  // persistent iterations of the solve graph (wl_persist.cuh)
+  // persistent iterations of wl_solve (wl_persist.cuh), for a solve with no other in flight on the device
   bool persist = false;
   unsigned* psync = nullptr;       // device: barrier arrivals of the current launch
   int* perr = nullptr;             // device: set when a barrier wait ran out
@@ -2076,7 +2084,8 @@ extern "C" void wl_engine_destroy(wl_engine* E) {
   cudaStream_t st = engine_stream(E);
   if (st) cudaStreamSynchronize(st);
   if (E->gexec) cudaGraphExecDestroy(E->gexec);
-  if (E->gloop) cudaGraphExecDestroy(E->gloop);
+  E->loop.release();
+  E->ploop.release();
   if (E->grun) cudaGraphExecDestroy(E->grun);
   IField* fs[] = {&E->b64, &E->x64, &E->y64, &E->t64, &E->xs, &E->rs, &E->p, &E->y, &E->t1};
   for (IField* f : fs) free_field(*f);
@@ -2399,13 +2408,15 @@ static wl_status build_graph(wl_engine* E, cudaStream_t st) {
   return WL_OK;
 }
 
-// The whole solve as one graph: a WHILE node whose body is one iteration, whose finalize
-// kernel (solve_loop_step) keeps the loop going while any slot is active and fewer than
-// `cap` iterations have run (a hard bound on the device loop; slots stop at their maxiter
-// long before).  wl_solve launches it once per solve instead of launching an iteration graph
-// and synchronising on a status poll every check_every iterations.  On any failure the
-// engine keeps the host-driven loop.
-static wl_status build_loop_graph(wl_engine* E, cudaStream_t st, bool run_mode = false) {
+// The whole solve as one graph: a WHILE node whose body is one iteration (E->loop) or one
+// persistent round (E->ploop), whose finalize kernel (solve_loop_step) keeps the loop going
+// while any slot is active and fewer than `cap` passes have run (a hard bound on the device
+// loop; slots stop at their maxiter long before).  wl_solve launches it once per solve instead
+// of launching an iteration graph and synchronising on a status poll every check_every
+// iterations.  On any failure the engine keeps the host-driven loop.  loop = null: the graph of
+// wl_engine_run.
+static wl_status build_loop_graph(wl_engine* E, cudaStream_t st, SolveLoopGraph* loop) {
+  const bool run_mode = loop == nullptr;
   wl_ctx* ctx = E->ctx;
   cudaGraph_t graph = nullptr;
   WL_CUDA(ctx, cudaGraphCreate(&graph, 0));
@@ -2425,19 +2436,19 @@ static wl_status build_loop_graph(wl_engine* E, cudaStream_t st, bool run_mode =
     if (e == cudaSuccess) body = cp.conditional.phGraph_out[0];
   }
   long long nk = 0;
+  int cap = 0;
+  for (int m : E->h_maxiter) cap = std::max(cap, m);
   if (e == cudaSuccess) {
-    int cap = 0;
-    for (int m : E->h_maxiter) cap = std::max(cap, m);
     SolveLoop L{E->n_active, E->loop_count, cap + 8, wh, nullptr, nullptr, nullptr};
     if (run_mode) L = SolveLoop{E->n_active, E->run_state + 2, 0, wh, E->run_state, E->run_state + 1, E->run_state + 3};
-    e = E->persist && !run_mode ? capture_persist(E, st, body, &L, &nk) : capture_iteration(E, st, body, &L, &nk);
+    e = loop == &E->ploop ? capture_persist(E, st, body, &L, &nk) : capture_iteration(E, st, body, &L, &nk);
   }
-  cudaGraphExec_t& exec = run_mode ? E->grun : E->gloop;
+  cudaGraphExec_t& exec = run_mode ? E->grun : loop->exec;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) {
     exec = nullptr;
-    (run_mode ? E->run_failed : E->loop_failed) = true;
+    (run_mode ? E->run_failed : loop->failed) = true;
     cudaGetLastError();
     return WL_ERR_CUDA;
   }
@@ -2445,9 +2456,9 @@ static wl_status build_loop_graph(wl_engine* E, cudaStream_t st, bool run_mode =
     E->run_kernels = nk;
     return WL_OK;
   }
-  E->loop_kernels = nk;
-  E->loop_cap = 0;
-  for (int m : E->h_maxiter) E->loop_cap = std::max(E->loop_cap, m);
+  loop->kernels = nk;
+  loop->cap = cap;
+  loop->gauge_id = E->gauge->id;
   return WL_OK;
 }
 
@@ -2466,7 +2477,7 @@ extern "C" wl_status wl_engine_run(wl_engine* E, int max_iters) {
     E->grun = nullptr;
   }
   if (!E->grun) {
-    if (build_loop_graph(E, st, true) != WL_OK) {
+    if (build_loop_graph(E, st, nullptr) != WL_OK) {
       ctx->err.clear();
       return wl_engine_step(E, max_iters);
     }
@@ -2730,55 +2741,56 @@ extern "C" wl_status wl_engine_retire(wl_engine* E, int slot, void* x, wl_solve_
 }
 
 // ------------------------------------------------------------------ solve
-// One launch of the engine's whole-solve graph (built on first use, rebuilt when the gauge or
-// the iteration limit changed); *ran is false when the graph is unavailable and the caller
-// drives the iterations from the host instead.
-// Persistent solves of one device take turns: two of them, each with a block per SM, could otherwise hold half of the
-// SMs each and wait for the other's blocks.  Held from the launch to the synchronisation that ends it.
-static std::mutex g_persist_mu[64];
-static std::unique_lock<std::mutex> persist_turn(const wl_engine* E) {
-  return E->persist ? std::unique_lock<std::mutex>(g_persist_mu[E->ctx->device & 63]) : std::unique_lock<std::mutex>();
-}
+// Solves in flight on a device, over all contexts and threads.  A persistent solve takes every SM whole, and two of them
+// could each hold half of the SMs and wait for the other's blocks; ordinary launches of several solves fill each
+// other's gaps.  So a solve takes the persistent form only if no other one is in flight when it starts, which also
+// means that there is at most one at a time.  Measured (B200, solves/s of 1 / 2 / 4 threads, each with its own context
+// and stream, for 12 FP16 slots at 8^4; FP32 at 12^3x24; FP64 at 8^4): persistent solves that take turns 356 / 376 /
+// 371; 157 / 161 / 165; 192 / 201 / 199; ordinary launches only 241 / 409 / 635; 125 / 202 / 295; 130 / 256 / 471; this
+// rule 366 / 412 / 644; 155 / 205 / 312; 193 / 283 / 498.
+static std::atomic<int> g_solving[64];
+struct SolveInFlight {
+  std::atomic<int>& count;
+  const bool alone;
+  explicit SolveInFlight(const wl_ctx* ctx)
+      : count(g_solving[ctx->device & 63]), alone(count.fetch_add(1) == 0) {}
+  ~SolveInFlight() { count.fetch_sub(1); }
+  SolveInFlight(const SolveInFlight&) = delete;
+};
 
 static const char* const kPersistTimeout = "a bounded device wait of the persistent iteration ran out";
 
-static wl_status run_loop_graph(wl_engine* E, bool* ran) {
+// One launch of the engine's whole-solve graph, over the ordinary iteration or the persistent round (built on first
+// use, rebuilt when the gauge or the iteration limit changed); *ran is false when the graph is unavailable, nothing
+// has run and the caller drives the iterations another way.
+static wl_status run_loop_graph(wl_engine* E, bool persist, bool* ran) {
   *ran = false;
-  if (E->loop_failed) return WL_OK;
+  SolveLoopGraph& L = persist ? E->ploop : E->loop;
+  if (L.failed) return WL_OK;
   wl_ctx* ctx = E->ctx;
   cudaStream_t st = engine_stream(E);
   int cap = 0;
   for (int m : E->h_maxiter) cap = std::max(cap, m);
-  if (E->gloop && (E->loop_gauge_id != E->gauge->id || E->loop_cap != cap)) {
-    cudaGraphExecDestroy(E->gloop);
-    E->gloop = nullptr;
-  }
-  const int n = E->n;
-  WL_CUDA(ctx, cudaMemsetAsync(E->loop_count, 0, sizeof(int), st));
-  const auto turn = persist_turn(E);
-  for (;;) {
-    cudaError_t e = cudaErrorNotSupported;
-    if (E->gloop || build_loop_graph(E, st) == WL_OK) {
-      E->loop_gauge_id = E->gauge->id;
-      e = cudaGraphLaunch(E->gloop, st);
-    }
-    if (e == cudaSuccess) break;
-    if (E->persist) {  // no cooperative kernel in a loop body here, and nothing ran: loop over the ordinary iteration
-      cudaGetLastError();
-      if (E->gloop) cudaGraphExecDestroy(E->gloop);
-      E->gloop = nullptr;
-      E->persist = E->loop_failed = false;
-      continue;
-    }
-    if (E->gloop) WL_CUDA(ctx, e);
+  if (L.gauge_id != E->gauge->id || L.cap != cap) L.release();
+  if (!L.exec && build_loop_graph(E, st, &L) != WL_OK) {
     ctx->err.clear();
     return WL_OK;
   }
+  const int n = E->n;
+  WL_CUDA(ctx, cudaMemsetAsync(E->loop_count, 0, sizeof(int), st));
+  const cudaError_t e = cudaGraphLaunch(L.exec, st);
+  if (e != cudaSuccess && persist) {  // the cooperative kernel is refused here
+    cudaGetLastError();
+    L.release();
+    L.failed = true;
+    return WL_OK;
+  }
+  WL_CUDA(ctx, e);
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 2 + n, E->loop_count, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 4 + n, E->perr, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaStreamSynchronize(st));
   if (E->h_pinned[4 + n]) WL_FAIL(ctx, WL_ERR_TIMEOUT, kPersistTimeout);
-  g_launches += (long long)E->h_pinned[2 + n] * E->loop_kernels;
+  g_launches += (long long)E->h_pinned[2 + n] * L.kernels;
   *ran = true;
   return WL_OK;
 }
@@ -2798,6 +2810,7 @@ extern "C" wl_status wl_solve(wl_ctx* ctx, wl_gauge* G, const wl_solve_params* p
   NvtxRange nvtx_range("wl_solve");
   if (!ctx || !G || !prm || !masses || !b || !x) WL_FAIL(ctx, WL_ERR_ARG, "null argument");
   if (nrhs <= 0) WL_FAIL(ctx, WL_ERR_ARG, "nrhs must be positive");
+  const SolveInFlight flight(ctx);
   wl_engine* E = nullptr;
   SolveKey key{ctx, prm->op, prm->inner_prec, nrhs, prm->use_graph};
   {
@@ -2822,9 +2835,9 @@ extern "C" wl_status wl_solve(wl_ctx* ctx, wl_gauge* G, const wl_solve_params* p
       E->gexec = nullptr;
       E->graph_built = false;
     }
-    if (E->gloop && delta_changed) {
-      cudaGraphExecDestroy(E->gloop);
-      E->gloop = nullptr;
+    if (delta_changed) {
+      E->loop.release();
+      E->ploop.release();
     }
   } else {
     wl_status s = wl_engine_create(ctx, G, prm, nrhs, &E);
@@ -2834,19 +2847,22 @@ extern "C" wl_status wl_solve(wl_ctx* ctx, wl_gauge* G, const wl_solve_params* p
   int n_active = 1;
   long long done_iters = 0;
   const int chunk = E->prm.check_every;
-  bool looped = false;
-  if (s == WL_OK && E->prm.use_graph) s = run_loop_graph(E, &looped);
+  bool persist = E->persist && flight.alone, looped = false;
+  if (s == WL_OK && E->prm.use_graph && persist) {
+    s = run_loop_graph(E, true, &looped);
+    if (s == WL_OK && !looped) E->persist = persist = false;
+  }
+  if (s == WL_OK && E->prm.use_graph && !looped) s = run_loop_graph(E, false, &looped);
   if (looped) s = wl_engine_poll(E, nullptr, &n_active);  // status, counters, wait errors
   while (s == WL_OK && !looped) {  // host-driven: the same rounds or iterations without the loop graph
     s = wl_engine_poll(E, nullptr, &n_active);
     if (s != WL_OK || n_active == 0) break;
     if (done_iters > (long long)E->prm.maxiter + 2 * chunk) break;  // host-side guard
-    if (E->persist) {
-      const auto turn = persist_turn(E);
+    if (persist) {
       const cudaError_t e = enqueue_persist_round(E, engine_stream(E), nullptr);
       int err = 0;
       if (e != cudaSuccess) {
-        E->persist = false;  // no cooperative launch here: step the iterations
+        E->persist = persist = false;  // no cooperative launch here: step the iterations
         cudaGetLastError();
       } else if (cudaMemcpyAsync(&err, E->perr, sizeof(int), cudaMemcpyDeviceToHost, engine_stream(E)) != cudaSuccess ||
                  cudaStreamSynchronize(engine_stream(E)) != cudaSuccess || err) {
