@@ -1617,6 +1617,15 @@ static int persist_mode() {
   return mode;
 }
 
+// WL_PERSIST_POLLS: another limit of a barrier wait (0: every wait that is not over at its first poll runs out)
+static int persist_polls() {
+  static const int polls = [] {
+    const char* e = std::getenv("WL_PERSIST_POLLS");
+    return e ? std::atoi(e) : kPersistPolls;
+  }();
+  return polls;
+}
+
 static bool persist_applies(const wl_engine* E) {
   const int mode = persist_mode();
   // a forced hop shape is forced for the ordinary launches
@@ -1697,6 +1706,7 @@ static cudaError_t enqueue_persist(wl_engine* E, cudaStream_t st) {
   A.partials = E->ppart;
   A.arrived = E->psync;
   A.err = E->perr;
+  A.polls = persist_polls();
   A.n = E->n;
   A.group = E->lanes_mode ? 1 : 0;
   cudaError_t e = cudaMemsetAsync(E->psync, 0, sizeof(unsigned), st);
@@ -2758,12 +2768,11 @@ struct SolveInFlight {
   SolveInFlight(const SolveInFlight&) = delete;
 };
 
-static const char* const kPersistTimeout = "a bounded device wait of the persistent iteration ran out";
-
 // One launch of the engine's whole-solve graph, over the ordinary iteration or the persistent round (built on first
 // use, rebuilt when the gauge or the iteration limit changed); *ran is false when the graph is unavailable, nothing
-// has run and the caller drives the iterations another way.
-static wl_status run_loop_graph(wl_engine* E, bool persist, bool* ran) {
+// has run and the caller drives the iterations another way.  *timeout: a wait of the persistent kernel ran out, and
+// the state of the solve is of no use.
+static wl_status run_loop_graph(wl_engine* E, bool persist, bool* ran, bool* timeout) {
   *ran = false;
   SolveLoopGraph& L = persist ? E->ploop : E->loop;
   if (L.failed) return WL_OK;
@@ -2789,10 +2798,49 @@ static wl_status run_loop_graph(wl_engine* E, bool persist, bool* ran) {
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 2 + n, E->loop_count, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaMemcpyAsync(E->h_pinned + 4 + n, E->perr, sizeof(int), cudaMemcpyDeviceToHost, st));
   WL_CUDA(ctx, cudaStreamSynchronize(st));
-  if (E->h_pinned[4 + n]) WL_FAIL(ctx, WL_ERR_TIMEOUT, kPersistTimeout);
+  *timeout = E->h_pinned[4 + n] != 0;
   g_launches += (long long)E->h_pinned[2 + n] * L.kernels;
   *ran = true;
   return WL_OK;
+}
+
+// The iterations of a solve, from admission on; *timeout as for run_loop_graph.
+static wl_status solve_once(wl_engine* E, const void* b, const void* x0, const double* masses, bool alone,
+                            bool* timeout) {
+  wl_ctx* ctx = E->ctx;
+  wl_status s = engine_admit_all(E, b, x0, masses);
+  int n_active = 1;
+  long long done_iters = 0;
+  const int chunk = E->prm.check_every;
+  bool persist = E->persist && alone, looped = false;
+  if (s == WL_OK && E->prm.use_graph && persist) {
+    s = run_loop_graph(E, true, &looped, timeout);
+    if (s == WL_OK && !looped) E->persist = persist = false;
+  }
+  if (s == WL_OK && E->prm.use_graph && !looped) s = run_loop_graph(E, false, &looped, timeout);
+  if (s == WL_OK && looped) s = wl_engine_poll(E, nullptr, &n_active);  // status, counters
+  while (s == WL_OK && !looped) {  // host-driven: the same rounds or iterations without the loop graph
+    s = wl_engine_poll(E, nullptr, &n_active);
+    if (s != WL_OK || n_active == 0) break;
+    if (done_iters > (long long)E->prm.maxiter + 2 * chunk) break;  // host-side guard
+    if (!persist) {
+      s = wl_engine_step(E, chunk);
+      done_iters += chunk;
+      continue;
+    }
+    if (enqueue_persist_round(E, engine_stream(E), nullptr) != cudaSuccess) {
+      E->persist = persist = false;  // no cooperative launch here: step the iterations
+      cudaGetLastError();
+      continue;
+    }
+    int err = 0;
+    WL_CUDA(ctx, cudaMemcpyAsync(&err, E->perr, sizeof(int), cudaMemcpyDeviceToHost, engine_stream(E)));
+    WL_CUDA(ctx, cudaStreamSynchronize(engine_stream(E)));
+    *timeout = err != 0;
+    if (*timeout) break;
+    done_iters += 1;
+  }
+  return s;
 }
 
 struct SolveKey {
@@ -2843,37 +2891,13 @@ extern "C" wl_status wl_solve(wl_ctx* ctx, wl_gauge* G, const wl_solve_params* p
     wl_status s = wl_engine_create(ctx, G, prm, nrhs, &E);
     if (s != WL_OK) return s;
   }
-  wl_status s = engine_admit_all(E, b, prm->use_x0 ? x : nullptr, masses);
-  int n_active = 1;
-  long long done_iters = 0;
-  const int chunk = E->prm.check_every;
-  bool persist = E->persist && flight.alone, looped = false;
-  if (s == WL_OK && E->prm.use_graph && persist) {
-    s = run_loop_graph(E, true, &looped);
-    if (s == WL_OK && !looped) E->persist = persist = false;
-  }
-  if (s == WL_OK && E->prm.use_graph && !looped) s = run_loop_graph(E, false, &looped);
-  if (looped) s = wl_engine_poll(E, nullptr, &n_active);  // status, counters, wait errors
-  while (s == WL_OK && !looped) {  // host-driven: the same rounds or iterations without the loop graph
-    s = wl_engine_poll(E, nullptr, &n_active);
-    if (s != WL_OK || n_active == 0) break;
-    if (done_iters > (long long)E->prm.maxiter + 2 * chunk) break;  // host-side guard
-    if (persist) {
-      const cudaError_t e = enqueue_persist_round(E, engine_stream(E), nullptr);
-      int err = 0;
-      if (e != cudaSuccess) {
-        E->persist = persist = false;  // no cooperative launch here: step the iterations
-        cudaGetLastError();
-      } else if (cudaMemcpyAsync(&err, E->perr, sizeof(int), cudaMemcpyDeviceToHost, engine_stream(E)) != cudaSuccess ||
-                 cudaStreamSynchronize(engine_stream(E)) != cudaSuccess || err) {
-        ctx->err = kPersistTimeout;
-        s = WL_ERR_TIMEOUT;
-      }
-      done_iters += 1;
-      continue;
-    }
-    s = wl_engine_step(E, chunk);
-    done_iters += chunk;
+  // x is written at the end, so a solve whose persistent form gave up starts again from the caller's data
+  bool timeout = false;
+  wl_status s = solve_once(E, b, prm->use_x0 ? x : nullptr, masses, flight.alone, &timeout);
+  if (s == WL_OK && timeout) {
+    E->persist = timeout = false;
+    s = cudaMemsetAsync(E->perr, 0, sizeof(int), engine_stream(E)) == cudaSuccess ? WL_OK : WL_ERR_CUDA;
+    if (s == WL_OK) s = solve_once(E, b, prm->use_x0 ? x : nullptr, masses, false, &timeout);
   }
   if (s == WL_OK) s = engine_unpack(E, 0, nrhs, x);
   std::vector<wl_solve_stats> tmp(nrhs);

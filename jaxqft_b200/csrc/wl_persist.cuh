@@ -16,8 +16,9 @@
 //
 // Barriers: one counter that every block increments once per barrier, zeroed before the launch; all blocks are
 // resident (cooperative launch, one block per SM).  Every wait has an iteration limit; a block whose wait runs out
-// sets *err, deactivates all slots and returns, so that the remaining waits run out too and the solve ends with an
-// error instead of hanging.
+// sets *err, deactivates all slots and returns, so that the remaining waits run out too.  Launches that find *err set
+// deactivate all slots and do nothing else, which ends the solve's loop; wl_solve then starts the solve again with the
+// ordinary launches.
 // Measured (B200, whole solves to 1e-12, ordinary launches -> this kernel): 12 point sources on 8^4 in FP16 3.97 ->
 // 2.66 ms (links staged every sweep 2.93), one even-odd FP32 solve at 16^3x32 10.8 -> 9.1 ms, plain FP64 CG at
 // 12^3x24 23.3 -> 20.4 ms, an MD update at 16^3x32 (full-lattice FP32 solve) 11.9 -> 8.6 ms.  What is left of an
@@ -29,7 +30,7 @@
 namespace wl {
 
 constexpr int kPersistMaxSlots = 16;
-constexpr int kPersistSpinLimit = 1 << 21;  // polls of one barrier wait (about a microsecond each)
+constexpr int kPersistPolls = 1 << 21;  // limit of the polls of one barrier wait (about a microsecond each)
 
 enum PersistKind { PK_SITE = 0, PK_PAIR = 1, PK_LANES = 2 };
 
@@ -50,6 +51,7 @@ struct PersistArgs {
   int* err;
   int n;             // slots, <= kPersistMaxSlots
   int group;
+  int polls;         // limit of one barrier wait
   int per;           // sites (PK_SITE, PK_PAIR: whole warps) or warp tiles (PK_LANES) per block
 };
 
@@ -63,7 +65,7 @@ struct PersistState {
 };
 
 // One grid barrier; false if its wait ran out.  `target`: arrivals expected by now (kept by the caller).
-WL_D bool grid_barrier(unsigned* arrived, unsigned& target, PersistState& st) {
+WL_D bool grid_barrier(unsigned* arrived, unsigned& target, int limit, PersistState& st) {
   target += gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -73,7 +75,7 @@ WL_D bool grid_barrier(unsigned* arrived, unsigned& target, PersistState& st) {
     int polls = 0;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
-    } while (seen < target && ++polls < kPersistSpinLimit);
+    } while (seen < target && ++polls < limit);
     st.go = seen >= target;
     __threadfence();
   }
@@ -327,9 +329,12 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
     st.maxiter[tid] = A.sc.maxiter[tid];
     st.status[tid] = A.sc.status[tid];
     st.ru[tid] = 0;
-    mine = st.active[tid] != 0;
+    mine = st.active[tid] != 0 && *A.err == 0;
   }
-  if (!__syncthreads_or(mine)) return;  // the same in every block
+  if (!__syncthreads_or(mine)) {  // nothing to solve, or a wait of an earlier launch ran out: the same in every block
+    if (tid < A.n) A.sc.active[tid] = A.sc.ru[tid] = 0;
+    return;
+  }
   const bool keep = KIND == PK_LANES && R >= 8 && EO && A.per <= T / 32;
   bool staged = false;  // the links of both parities are in shared memory (from the second iteration on)
   const auto hop = [&](auto dag, const SF(&src)[2], int parity0, int np, const auto& epi, double* partials) {
@@ -349,24 +354,24 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
     // ---- y = M p (or D p), pAp = |y|^2
     if constexpr (EO) {
       hop(plain, A.p, 1, 1, A.et, nullptr);
-      if (!(ok = grid_barrier(A.arrived, target, st))) break;
+      if (!(ok = grid_barrier(A.arrived, target, A.polls, st))) break;
       hop(plain, A.t1, 0, 1, A.ey, part0);
     } else {
       hop(plain, A.p, 0, 2, A.ey, part0);
     }
-    if (!(ok = grid_barrier(A.arrived, target, st))) break;
+    if (!(ok = grid_barrier(A.arrived, target, A.polls, st))) break;
     persist_sum(part0, A.n, st, st.pap);
     if (tid < A.n && st.active[tid]) A.alpha[tid] = st.pap[tid] > 0.0 ? st.r2[tid] / st.pap[tid] : 0.0;
     __syncthreads();
     // ---- x_s += alpha p, r_s -= alpha M^dag y, r2n = |r_s|^2
     if constexpr (EO) {
       hop(dagger, A.y, 1, 1, A.et, nullptr);
-      if (!(ok = grid_barrier(A.arrived, target, st))) break;
+      if (!(ok = grid_barrier(A.arrived, target, A.polls, st))) break;
       hop(dagger, A.t1, 0, 1, A.ec, part1);
     } else {
       hop(dagger, A.y, 0, 2, A.ec, part1);
     }
-    if (!(ok = grid_barrier(A.arrived, target, st))) break;
+    if (!(ok = grid_barrier(A.arrived, target, A.polls, st))) break;
     persist_sum(part1, A.n, st, st.r2n);
     // ---- decision and bookkeeping (cg_decide_kernel, cg_finalize_kernel), the same in every block
     bool trig = false, live = false;
@@ -394,9 +399,9 @@ __global__ void __launch_bounds__(T, 1) cg_persist_kernel(const __grid_constant_
     }
     __syncthreads();
     sweep_update<KIND, R>(A, npar, st, SF{});
-    if (!(ok = grid_barrier(A.arrived, target, st))) break;
+    if (!(ok = grid_barrier(A.arrived, target, A.polls, st))) break;
   }
-  if (!ok) {  // a wait ran out: stop the solve
+  if (!ok) {  // a wait ran out: stop the solve (this launch's stores to the state are not used)
     if (tid < A.n) {
       A.sc.active[tid] = 0;
       A.sc.ru[tid] = 0;
