@@ -279,7 +279,7 @@ wl_status wl_pf_force_eo(wl_ctx* ctx, wl_gauge* gauge, const void* X, const void
    (jaxqft/models/su3_ym.py:298-327 _staple / force_reference; su3_ym.py:96-123
    the BMXYIJ form).  F has U's shape. */
 wl_status wl_gauge_force(wl_ctx* ctx, const void* U, int batch, double beta, void* F);
-/* the same with the caller's scratch of the size of U (NULL: the context's own, allocated on first use) */
+/* the same; `scratch` is not used and may be NULL (kept for callers that pass one) */
 wl_status wl_gauge_force_ws(wl_ctx* ctx, const void* U, int batch, double beta, void* scratch, void* F);
 
 /* Uout = exp(dt P) U per link (su3_ym.py:349-350 evolve_q_reference with

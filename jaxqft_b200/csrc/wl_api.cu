@@ -1064,26 +1064,18 @@ static GaugeArgs gauge_args(wl_ctx* ctx, const void* U, const void* P, void* out
   return A;
 }
 
-extern "C" wl_status wl_gauge_force_ws(wl_ctx* ctx, const void* U, int batch, double beta, void* scratch, void* F) {
+extern "C" wl_status wl_gauge_force(wl_ctx* ctx, const void* U, int batch, double beta, void* F) {
   NvtxRange nvtx_range("wl_gauge_force");
   if (!ctx || !U || !F || batch < 1) WL_FAIL(ctx, WL_ERR_ARG, "null argument or batch < 1");
   WL_CUDA(ctx, cudaSetDevice(ctx->device));
-  const Geom& g = ctx->g;
-  if (!scratch) {
-    wl_status s = ensure_tmp(ctx, (size_t)batch * 4 * g.V * 9 * sizeof(double2));
-    if (s != WL_OK) return s;
-    scratch = ctx->tmp;
-  }
-  g_launches += 2;
-  gauge_soa_kernel<<<dim3((g.V + 127) / 128, 4, batch), 128, 0, ctx->stream>>>((const double2*)U, (double2*)scratch,
-                                                                              g.V);
-  GaugeArgs A = gauge_args(ctx, scratch, nullptr, F, batch, -beta / 3.0);
-  gauge_force_kernel<<<dim3((g.V + 31) / 32, 1, batch), 128, 0, ctx->stream>>>(A);
+  GaugeArgs A = gauge_args(ctx, U, nullptr, F, batch, -beta / 3.0);
+  g_launches++;
+  gauge_force_kernel<<<dim3((ctx->g.V + 31) / 32, 1, batch), 128, 0, ctx->stream>>>(A);
   return check_launch(ctx, "gauge_force_kernel");
 }
 
-extern "C" wl_status wl_gauge_force(wl_ctx* ctx, const void* U, int batch, double beta, void* F) {
-  return wl_gauge_force_ws(ctx, U, batch, beta, nullptr, F);
+extern "C" wl_status wl_gauge_force_ws(wl_ctx* ctx, const void* U, int batch, double beta, void*, void* F) {
+  return wl_gauge_force(ctx, U, batch, beta, F);
 }
 
 extern "C" wl_status wl_gauge_evolve(wl_ctx* ctx, const void* P, const void* U, int batch, double dt, void* Uout) {

@@ -209,49 +209,17 @@ WL_D void m3_lds(M3& a, const double2* p) {
 }
 
 // ---------------------------------------------------------------- force
-// Two kernels.  The links arrive as 144-byte matrices; read in place, a warp's 16-byte load spans 36 lines, and at
-// 171 such loads a link the L1 pipe took the whole 174 us of the kernel this replaced (16^3x32).  So the links are
-// first copied to a matrix-element-major scratch, [batch][mu][9][V] double2, through shared memory (both sides
-// contiguous; 25 us), where the same loads are 512 contiguous bytes.
-//
-// gauge_force_kernel: one thread per link.  A block is 32 consecutive sites with one warp per direction, so that the
-// 76 link reads of a site (31 distinct ones per row) meet in L1.  Bound by the latency of those reads at 12 warps
-// per SM (168 registers: three matrices and the staple sum live) next to 1404 FP64 FMAs a link.
-// Measured at 16^3x32: force and drift together 270 -> 220 us on new links each call (floor 47 us of DRAM, 40 us of
-// FP64); on the same links each call the force takes 25 + 113 us against 174 us.  168 registers (3 blocks) 113 us, 8 warps
-// 139 us, 128 registers (spills) 147 us.  Also measured and not kept: the 31 rows of a 16-site segment staged in
-// shared memory with 18 threads a site (215 us: two phase-locked blocks per SM), 8-site segments (234 us), and 4D
-// site tiles per block (117-152 us).
-__global__ void __launch_bounds__(128) gauge_soa_kernel(const double2* __restrict__ src, double2* __restrict__ dst,
-                                                        int V) {
-  __shared__ double2 sm[4][32 * 9];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int f0 = (int)(blockIdx.x * 4 + warp) * 32;
-  if (f0 >= V) return;  // uniform per warp; only warp barriers below
-  const int n = min(32, V - f0);
-  const size_t plane = (size_t)blockIdx.z * 4 + blockIdx.y;  // (configuration, direction)
-  const double2* s = src + (plane * V + f0) * 9;
-  for (int q = lane; q < n * 9; q += 32) cp16(&sm[warp][q], s + q);
-  cp16_wait();
-  __syncwarp();
-  if (lane < n) {
-    double2* o = dst + plane * 9 * V + f0 + lane;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) o[(size_t)k * V] = sm[warp][lane * 9 + k];
-  }
-}
-
-// element k of the link of direction mu at flat site f: base + (mu * 9 + k) * V + f
-WL_D void m3_load_soa(M3& a, const double2* base, int V, int mu, int f) {
-  const double2* p = base + (size_t)mu * 9 * V + f;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const double2 v = ldg(p + (size_t)k * V);
-    a.m[k / 3][k % 3] = {v.x, v.y};
-  }
-}
-
-// A.U: the scratch of gauge_soa_kernel.  grid: x over groups of 32 sites, z = batch
+// One thread per link.  A block is 32 consecutive sites with one warp per direction, so that the 76 link reads of a
+// site (31 distinct ones per row) meet in L1; the 32 results of a warp are staged in shared memory and leave as one
+// contiguous 4608-byte run.  162 registers (three matrices and the staple sum live) leave 12 warps per SM; next to the
+// reads, 144-byte matrices in 16-byte loads, stand 1404 FP64 FMAs a link.
+// Measured (B200, us of the force alone, three prepared configurations in turn) against blocks of 128 sites of one
+// direction with unstaged stores: 8^4 10.3 -> 10.3 (the host's share), 12^3x24 55.5 -> 53.4, 16^3x32 174 -> 157
+// (floor 24 us of DRAM, 40 us of FP64), three configurations of 16^3x32 515 -> 458.  Also measured and not kept: the
+// links copied first to a matrix-element-major scratch, whose reads are contiguous (15.4, 55.1, 159, 469 us: the copy
+// takes what the reads save); the 31 rows of a 16-site segment staged in shared memory with 18 threads a site; 4D site
+// tiles per block.
+// grid: x over groups of 32 sites, z = batch
 __global__ void __launch_bounds__(128, 3) gauge_force_kernel(GaugeArgs A) {
   __shared__ double2 sm[4][32 * 9];
   const Geom& g = A.g;
@@ -259,8 +227,9 @@ __global__ void __launch_bounds__(128, 3) gauge_force_kernel(GaugeArgs A) {
   const int f0 = (int)blockIdx.x * 32, f = f0 + lane;
   const size_t plane = (size_t)blockIdx.z * 4;
   if (f < g.V) {
-    const double2* S = A.U + plane * 9 * g.V;
+    const double2* links = A.U + plane * 9 * g.V;
     const Site s = site_of_flat(g, f);
+    const auto load = [&](M3& a, int dir, int site) { m3_load(a, links + ((size_t)dir * g.V + site) * 9); };
     const auto at = [&](int mu1, int d1, int mu2, int d2) { return (int)gshift(g, s.x, mu1, d1, mu2, d2); };
     M3 st, t, u, v;
 #pragma unroll
@@ -271,10 +240,10 @@ __global__ void __launch_bounds__(128, 3) gauge_force_kernel(GaugeArgs A) {
     for (int n = 1; n < 4; ++n) {
       const int nu = (mu + n) & 3;
       // forward: U_nu(x) U_mu(x+nu) U_nu(x+mu)^dag
-      m3_load_soa(u, S, g.V, nu, f);
-      m3_load_soa(v, S, g.V, mu, at(nu, +1, mu, 0));
+      load(u, nu, f);
+      load(v, mu, at(nu, +1, mu, 0));
       m3_mul(u, v, t);
-      m3_load_soa(u, S, g.V, nu, at(mu, +1, nu, 0));
+      load(u, nu, at(mu, +1, nu, 0));
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -283,10 +252,10 @@ __global__ void __launch_bounds__(128, 3) gauge_force_kernel(GaugeArgs A) {
           for (int k = 0; k < 3; ++k) fmac_(st.m[i][j], u.m[j][k], t.m[i][k]);
       // backward: U_nu(x-nu)^dag U_mu(x-nu) U_nu(x-nu+mu)
       const int fm = at(nu, -1, mu, 0);
-      m3_load_soa(u, S, g.V, nu, fm);
-      m3_load_soa(v, S, g.V, mu, fm);
+      load(u, nu, fm);
+      load(v, mu, fm);
       m3_mul_dn(u, v, t);
-      m3_load_soa(u, S, g.V, nu, at(nu, -1, mu, +1));
+      load(u, nu, at(nu, -1, mu, +1));
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -294,7 +263,7 @@ __global__ void __launch_bounds__(128, 3) gauge_force_kernel(GaugeArgs A) {
 #pragma unroll
           for (int k = 0; k < 3; ++k) fma_(st.m[i][j], t.m[i][k], u.m[k][j]);
     }
-    m3_load_soa(u, S, g.V, mu, f);
+    load(u, mu, f);
     m3_mul_nd(u, st, t);  // U_mu(x) V^dag
     m3_ta(t, v, A.coef);
 #pragma unroll

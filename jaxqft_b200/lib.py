@@ -330,8 +330,7 @@ class WilsonContext:
         U, B = self._links(U, "U")
         if out is None:
             out = torch.empty_like(U)
-        scratch = self._scratch(*U.shape)  # element-major copy of the links
-        self._check(self.lib.wl_gauge_force_ws(self.handle, _ptr(U), B, float(beta), _ptr(scratch), _ptr(out)))
+        self._check(self.lib.wl_gauge_force(self.handle, _ptr(U), B, float(beta), _ptr(out)))
         return out
 
     def gauge_evolve(self, dt: float, P, U, out=None):
