@@ -1586,12 +1586,15 @@ static void enqueue_iteration(wl_engine* E, cudaStream_t st, int part) {
 //   FP32 sites (1-3 slots): 14 (8^4, even-odd) 3.8 -> 3.1; 140 (12^3x24) 7.5 -> 5.9; 280 17.5 -> 10.9; 443 (16^3x32)
 //     10.8 -> 9.1; 886 31.5 -> 22.6, two slots 62.8 -> 45.1; beyond: 1081 (20^3x40) 27.3 -> 26.7, 2242 (24^3x48)
 //     51 -> 54.  FP16 sites: 443 12.3 -> 10.4; beyond: 1081 23.4 -> 23.9, 2242 48 -> 54
+//     FP16 even-odd solves of two and three slots only up to 640: 636 105 -> 103 and 120 -> 122, but 899 (16^2x20x52)
+//     159 -> 167 and 204 -> 220 (one slot 80 -> 72; full operator, 886: 345 -> 276 and 467 -> 403)
 //   FP64 pairs, by sites: 28 (8^4, full) 7.3 -> 5.6; 280 23.4 -> 20.3, two slots 46.2 -> 35.9; beyond: 443 20.7 -> 30.2
 //     Two and three slots only while each of the block's 12 warps gets one item (190 sites x slots a SM): beyond, a
 //     second, part-empty sweep made them 0.81-1.15 of the ordinary time (74 x 3: 5.1 -> 6.4; 91 x 3: 12.5 -> 10.9).
 //   FP16 lanes, by tiles: 7 (8^4, 12 slots) 4.0 -> 2.7; 18 (12^3x24) 11.0 -> 10.4; 35 22.0 -> 21.0; 55 28.6 -> 26.0
 //   FP32 lanes, by tiles: 7 4.3 -> 2.8; 35 32.3 -> 26.7; 110 108 -> 90; 140 92 -> 82
-constexpr int kPersistSites = 900, kPersistSitesD = 300, kPersistSlotSitesD = 190, kPersistTilesH = 60, kPersistTilesS = 150;
+constexpr int kPersistSites = 900, kPersistSitesH = 640, kPersistSitesD = 300, kPersistSlotSitesD = 190;
+constexpr int kPersistTilesH = 60, kPersistTilesS = 150;
 
 static long long persist_items(const wl_engine* E) {
   const long long vh = E->ctx->g.Vh;
@@ -1628,6 +1631,9 @@ static bool persist_applies(const wl_engine* E) {
   const long long most = E->lanes_mode ? (E->sprec == P_HALF ? kPersistTilesH : kPersistTilesS)
                                        : (E->sprec == P_DOUBLE ? kPersistSitesD : kPersistSites);
   if (mode == 2) return true;
+  if (!E->lanes_mode && E->sprec == P_HALF && E->n > 1 && E->prm.op == WL_SOLVE_EO_NORMAL &&
+      persist_items(E) > (long long)kPersistSitesH * E->ctx->sm_count)
+    return false;
   if (!E->lanes_mode && E->sprec == P_DOUBLE && E->n > 1 &&
       persist_items(E) * E->n > (long long)kPersistSlotSitesD * E->ctx->sm_count)
     return false;
