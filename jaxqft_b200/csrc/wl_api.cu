@@ -1209,16 +1209,16 @@ struct wl_engine {
   const SolveLoop* capture_loop = nullptr;  // set while part 3 of a loop body is captured
   // engine run (wl_engine_run): WHILE node that stops when a slot finishes or at a per-launch cap
   cudaGraphExec_t grun = nullptr;
-  int* run_state = nullptr;        // device: [0] cap, [1] active count at launch start, [2] iterations
+  int* run_state = nullptr;        // device: [0] cap, [1] active count at launch start, [2] iterations, [3] in all
   long long run_kernels = 0;       // unconditional kernels per run iteration
   long long run_seen = 0;          // run iterations already counted into g_launches
   unsigned long long run_gauge_id = 0;
   bool run_failed = false;
   // persistent iterations of wl_solve (wl_persist.cuh), for a solve with no other in flight on the device
   bool persist = false;
-  unsigned* psync = nullptr;       // device: barrier arrivals of the current launch
-  int* perr = nullptr;             // device: set when a barrier wait ran out
-  double* ppart = nullptr;         // device: [2][n][blocks] partial sums
+  unsigned* psync = nullptr;       // barrier arrivals of the current launch (behind run_state)
+  int* perr = nullptr;             // set when a barrier wait ran out (behind run_state)
+  double* ppart = nullptr;         // [2][n][blocks] partial sums (behind partials)
   bool ru_links12 = false;         // FP64 true residual with 12-real links (links unitary to 1e-12)
 };
 
@@ -2104,9 +2104,6 @@ extern "C" void wl_engine_destroy(wl_engine* E) {
   cudaFree(E->ru_iters);
   cudaFree(E->loop_count);
   cudaFree(E->run_state);
-  cudaFree(E->psync);
-  cudaFree(E->perr);
-  cudaFree(E->ppart);
   if (E->h_pinned) cudaFreeHost(E->h_pinned);
   if (E->poll_ev) cudaEventDestroy(E->poll_ev);
   if (st) cudaStreamDestroy(st);
@@ -2188,16 +2185,13 @@ extern "C" wl_status wl_engine_create(wl_ctx* ctx, wl_gauge* G, const wl_solve_p
   // most partial sums per RHS: one per warp of the RHS-in-lanes kernels; at 16 lanes a
   // warp covers 2 sites, so both parities give up to Vh partials
   const size_t nblk = (size_t)g.Vh + 64;
-  if (e == cudaSuccess) e = cudaMalloc(&E->partials, sizeof(double) * nblk * n);
+  const size_t npp = n <= kPersistMaxSlots ? (size_t)2 * n * ctx->sm_count : 0;
+  if (e == cudaSuccess) e = cudaMalloc(&E->partials, sizeof(double) * (nblk * n + npp));
   if (e == cudaSuccess) e = cudaMalloc(&E->counters, sizeof(unsigned) * (n + 1));
   if (e == cudaSuccess) e = cudaMallocHost(&E->h_pinned, sizeof(int) * (3 * n + 4));
   if (e == cudaSuccess) e = cudaMalloc(&E->ru_iters, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&E->loop_count, sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&E->run_state, 4 * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&E->psync, sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMalloc(&E->perr, sizeof(int));
-  if (e == cudaSuccess && n <= kPersistMaxSlots)
-    e = cudaMalloc(&E->ppart, sizeof(double) * 2 * n * ctx->sm_count);
+  if (e == cudaSuccess) e = cudaMalloc(&E->run_state, 6 * sizeof(int));
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&E->poll_ev, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     ctx->err = std::string("engine allocation: ") + cudaGetErrorString(e);
@@ -2208,8 +2202,10 @@ extern "C" wl_status wl_engine_create(wl_ctx* ctx, wl_gauge* G, const wl_solve_p
   cudaMemsetAsync(E->ints, 0, sizeof(int) * (kEngineInts * n + 1), st);
   cudaMemsetAsync(E->counters, 0, sizeof(unsigned) * (n + 1), st);
   cudaMemsetAsync(E->ru_iters, 0, sizeof(int), st);
-  cudaMemsetAsync(E->run_state, 0, 4 * sizeof(int), st);
-  cudaMemsetAsync(E->perr, 0, sizeof(int), st);
+  cudaMemsetAsync(E->run_state, 0, 6 * sizeof(int), st);
+  E->psync = (unsigned*)E->run_state + 4;
+  E->perr = E->run_state + 5;
+  E->ppart = E->partials + nblk * n;
   double* d = E->dbl;
   E->r2 = d + 0 * n; E->r2_new = d + 1 * n; E->pAp = d + 2 * n; E->r2_true = d + 3 * n;
   E->rmax2 = d + 4 * n; E->b2 = d + 5 * n; E->tol2 = d + 6 * n; E->beta = d + 7 * n;
