@@ -1612,6 +1612,15 @@ static int persist_mode() {
   return mode;
 }
 
+// WL_PERSIST_BLOCKS: at most this many blocks, so that a small lattice gives a warp several items (tests)
+static int persist_blocks(int sm_count) {
+  static const int most = [] {
+    const char* e = std::getenv("WL_PERSIST_BLOCKS");
+    return e ? std::max(1, std::atoi(e)) : 1 << 30;
+  }();
+  return std::min(most, sm_count);
+}
+
 // WL_PERSIST_POLLS: another limit of a barrier wait (0: every wait that is not over at its first poll runs out)
 static int persist_polls() {
   static const int polls = [] {
@@ -1650,8 +1659,8 @@ static cudaError_t launch_persist(wl_engine* E, PersistArgs<S, typename SloppyLi
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const long long items = persist_items(E);
-  const int sms = E->ctx->sm_count;
-  long long per = (items + sms - 1) / sms;
+  const int blocks = persist_blocks(E->ctx->sm_count);
+  long long per = (items + blocks - 1) / blocks;
   if (KIND != PK_LANES) {  // whole warps of sites
     const int w = KIND == PK_PAIR ? 16 : 32;
     per = (per + w - 1) / w * w;

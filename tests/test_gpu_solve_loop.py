@@ -4,7 +4,15 @@ than the iteration limit plus a few).  wl_engine_run uses the same loop, stoppin
 as a slot finishes.  Their results must be the host-driven iteration's: the same kernels
 in the same order, so bitwise the same solutions, iteration counts and statuses, for
 converged solves and for solves stopped at maxiter, and for slots that converge at
-different iterations."""
+different iterations.
+
+At this lattice's size wl_solve's loop runs the persistent rounds, from the graph and from
+the host; the last test runs the same assertions in a child process with WL_PERSIST=0, where
+the loop runs the ordinary iteration that larger solves and more than 16 slots take."""
+
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -108,3 +116,11 @@ def test_engine_run_stops_when_a_slot_finishes(setup, inner, nslots):
         s = W.schur_even(U, x, masses[r], bc, normalized=True)
         ax = W.schur_even(U, s, masses[r], bc, normalized=True, dag=True)[0]
         assert np.linalg.norm(b[r] - ax) / np.linalg.norm(b[r]) <= 1e-10
+
+
+@pytest.mark.skipif(os.environ.get("WL_PERSIST") == "0", reason="the child process of this test")
+def test_loop_graph_over_the_ordinary_iteration():
+    res = subprocess.run([sys.executable, "-m", "pytest", os.path.abspath(__file__), "-q", "-m", "gpu", "-k", "host_loop or maxiter"],
+                         capture_output=True, text=True, timeout=900, env=dict(os.environ, WL_PERSIST="0"),
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert res.returncode == 0 and "7 passed" in res.stdout, res.stdout[-3000:] + res.stderr[-2000:]
