@@ -27,11 +27,6 @@ WL_D void m3_load(M3& a, const double2* p) {
   }
 }
 
-WL_D void m3_store(const M3& a, double2* p) {
-#pragma unroll
-  for (int k = 0; k < 9; ++k) p[k] = make_double2(a.m[k / 3][k % 3].re, a.m[k / 3][k % 3].im);
-}
-
 // c = a b ; c = a b^dag ; c = a^dag b
 WL_D void m3_mul(const M3& a, const M3& b, M3& c) {
 #pragma unroll

@@ -25,7 +25,7 @@
 //
 // Bound by the L1 data pipe (79 % of its wavefront rate at 50 % of DRAM bandwidth at 24^3x48): every spinor load of
 // a warp touches one 64-byte piece of each of its 16 sites, and every link is delivered to both threads of a pair.
-// Measured (B200, new buffers each call) against warps of 16 consecutive flat sites, whose link loads are two
+// Measured (B200, three prepared states in turn) against warps of 16 consecutive flat sites, whose link loads are two
 // half-used runs, in blocks of 128 threads with separate memsets: S_e^dag S_e of three fields at 6x10x14x18 51.3 ->
 // 43.0 us, D at 24^3x48 201 -> 198 us, D^dag of 12 fields at 16^3x32 unchanged (415 us), D at 8^4 unchanged.  On the
 // same buffers every call: D at 24^3x48 187 -> 174 us, three fields at 6x10x14x18 19.6 -> 16.8 us.

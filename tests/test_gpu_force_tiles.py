@@ -1,9 +1,9 @@
-"""Force and gauge-sector kernels at the sizes where their tiling can go wrong: rows shorter than, equal to and
-ragged against the 16-site segments of the gauge force and the 64-site blocks of the pseudofermion force, extents
-of two (both neighbours the same site), fields that are not 32-byte aligned, accumulation, in-place drift.
+"""Force and gauge-sector kernels at the sizes where their tiling can go wrong: lattices smaller than, filling and ragged
+against the 32-site blocks of the gauge force and the 64-site blocks of the pseudofermion force, extents of two (both
+neighbours the same site), fields that are not 32-byte aligned, accumulation, in-place drift.
 
 Oracle: the numpy restatement.  Tolerances: every force entry is a sum of fewer than 200 products of numbers of
-order one in FP64, so a relative 2-norm error of 1e-13 leaves a factor of more than four over the worst case
+order one in FP64, so a relative 2-norm error of 1e-13 leaves a factor of more than two over the worst case
 200 eps; the drift squares s ~ log2 ||dt P|| times, each doubling the relative error of a few eps."""
 
 import numpy as np
@@ -20,7 +20,7 @@ if not torch.cuda.is_available():  # pragma: no cover
 from jaxqft_b200.lib import WilsonContext  # noqa: E402
 from jaxqft_b200.su3_wilson_nf2 import SU3WilsonNf2  # noqa: E402
 
-SHAPES = [(2, 2, 2, 2), (2, 4, 6, 16), (4, 2, 2, 18), (2, 2, 4, 34), (6, 2, 4, 10)]
+SHAPES = [(2, 2, 2, 2), (2, 4, 6, 16), (4, 2, 2, 18), (2, 2, 4, 34), (6, 2, 4, 10), (2, 6, 2, 10)]
 BC = (1, 1j, 1, -1)
 
 
