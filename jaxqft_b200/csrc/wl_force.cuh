@@ -27,10 +27,11 @@
 // site, and each of the two forces keeps the products in which its odd field meets the
 // other's even one.  X[p] / Y[p] are therefore separate pointers per site parity.
 //
-// Bound by the L1 data pipe and, next to it, by DRAM (each link read and written once,
-// each field once: 1536 bytes per site).  The kernel it replaced (one thread per link, AoS
-// links and spinors in 16-byte loads 144 and 192 bytes apart, 186 registers) spent
-// 80 % of the L1 pipe on those strides.
+// Bound by the latency of its loads at 16 warps per SM (128 registers): at 16^3x32 the L1 data
+// pipe is 65 % busy, DRAM runs at 2.9 TB/s (178 MB for 1536 bytes per site, each link read and
+// written once, each field once) and a warp waits for a load on 3 of 8 cycles between its
+// instructions.  The kernel it replaced (one thread per link, AoS links and spinors in 16-byte
+// loads 144 and 192 bytes apart, 186 registers) spent 80 % of the L1 pipe on those strides.
 // Measured (B200): 2 x 12^3x24 force 102 -> 45 us (floor 20 us at the measured copy rate), even-odd force at
 // 16^3x32, with its two hops, 368 -> 120 us (floor 27 us).
 #pragma once

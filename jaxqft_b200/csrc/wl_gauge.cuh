@@ -206,8 +206,9 @@ WL_D void m3_lds(M3& a, const double2* p) {
 // ---------------------------------------------------------------- force
 // One thread per link.  A block is 32 consecutive sites with one warp per direction, so that the 76 link reads of a
 // site (31 distinct ones per row) meet in L1; the 32 results of a warp are staged in shared memory and leave as one
-// contiguous 4608-byte run.  162 registers (three matrices and the staple sum live) leave 12 warps per SM; next to the
-// reads, 144-byte matrices in 16-byte loads, stand 1404 FP64 FMAs a link.
+// contiguous 4608-byte run.  Bound by the L1 data pipe: the reads are 144-byte matrices in 16-byte loads, which keep it
+// 86 % busy at 16^3x32 (60 % of their sectors hit), next to 1404 FP64 FMAs a link (FP64 pipe 40 %).  162 registers
+// (three matrices and the staple sum live) leave 12 warps per SM.
 // Measured (B200, us of the force alone, three prepared configurations in turn) against blocks of 128 sites of one
 // direction with unstaged stores: 8^4 10.3 -> 10.3 (the host's share), 12^3x24 55.5 -> 53.4, 16^3x32 174 -> 157
 // (floor 24 us of DRAM, 40 us of FP64), three configurations of 16^3x32 515 -> 458.  Also measured and not kept: the
