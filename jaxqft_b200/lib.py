@@ -239,18 +239,18 @@ class WilsonContext:
         self._stream = int(stream.cuda_stream)
         self._check(self.lib.wl_ctx_set_stream(self.handle, ctypes.c_void_p(self._stream)))
 
-    def _scratch(self, *shape):
-        """Uninitialised complex128 scratch that may be dropped while kernels of this context still use it: a block of
-        the context's stream, which the caching allocator gives only to work queued behind them.  (A block of another
-        current stream would be free for that stream's next tensor as soon as it is dropped.)"""
+    def _scratch(self, n):
+        """n uninitialised complex128 elements of scratch that may be dropped while kernels of this context still use
+        it: a block of the context's stream, which the caching allocator gives only to work queued behind them.  (A
+        block of another current stream would be free for that stream's next tensor as soon as it is dropped.)"""
         torch = self._torch
-        make = lambda: torch.empty(shape, dtype=torch.complex128, device=self.device)  # noqa: E731
-        if torch.cuda.current_stream(self.device).cuda_stream == self._stream:
-            return make()
+        # the handle alone: a Stream object costs 2 us, a third of the host time of a small force
+        if torch._C._cuda_getCurrentRawStream(self._index) == self._stream:
+            return torch.empty(n, dtype=torch.complex128, device=self.device)
         own = (torch.cuda.ExternalStream(self._stream, device=self.device) if self._stream
                else torch.cuda.default_stream(self.device))
         with torch.cuda.stream(own):
-            return make()
+            return torch.empty(n, dtype=torch.complex128, device=self.device)
 
     def _check(self, rc: int):
         if rc != WL_OK:
@@ -287,7 +287,10 @@ class WilsonContext:
 
     def _one_field(self, x, name):
         """One spinor field of the whole lattice as the force kernels read it: complex128, contiguous, on this device."""
-        x = _c128(x, self.device)
+        torch = self._torch
+        if not (type(x) is torch.Tensor and x.dtype is torch.complex128 and x.get_device() == self._index
+                and x.is_contiguous()):
+            x = _c128(x, self.device)
         if x.numel() != self._field:
             raise ValueError(f"{name} of {x.numel()} elements is not one field on lattice {self.lattice_shape}")
         return x
@@ -309,11 +312,13 @@ class WilsonContext:
         eo_coef; fields of one configuration, F (complex128, contiguous, on this device) overwritten."""
         X, Y = self._one_field(X, "X"), self._one_field(Y, "Y")
         if eo_coef is None:
-            self._check(self.lib.wl_pf_force(self.handle, gauge.handle, _ptr(X), _ptr(Y), 1.0, 0, _ptr(F)))
-            return
-        scratch = self._scratch(2, *self.lattice_shape, 4, 3)
-        self._check(self.lib.wl_pf_force_eo(self.handle, gauge.handle, _ptr(X), _ptr(Y), float(eo_coef),
-                                            _ptr(scratch), _ptr(F)))
+            rc = self.lib.wl_pf_force(self.handle, gauge.handle, X.data_ptr(), Y.data_ptr(), 1.0, 0, F.data_ptr())
+        else:
+            scratch = self._scratch(2 * self._field)
+            rc = self.lib.wl_pf_force_eo(self.handle, gauge.handle, X.data_ptr(), Y.data_ptr(), eo_coef,
+                                         scratch.data_ptr(), F.data_ptr())
+        if rc:
+            self._check(rc)
 
     # ------------------------------------------------------------ gauge sector
     def _links(self, x, name):
