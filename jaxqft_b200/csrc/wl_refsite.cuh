@@ -23,12 +23,15 @@
 // cf = -1 (D) or +1 (D^dag), cb = -cf, boundary phase on the forward hop from
 // x_mu = L_mu - 1 and (conjugated) on the backward hop into x_mu = 0.
 //
-// Bound by the L1 data pipe (79 % of its wavefront rate at 50 % of DRAM bandwidth at 24^3x48): every spinor load of
-// a warp touches one 64-byte piece of each of its 16 sites, and every link is delivered to both threads of a pair.
+// Bound by the latency of its loads at 14 warps per SM next to the L1 data pipe: at 16^3x32 (one field) a warp waits
+// for a load on 5.4 of 8.8 cycles between its instructions, the pipe is 63 % busy and DRAM runs at 2.75 TB/s.  Every
+// spinor load of a warp touches one 64-byte piece of each of its 16 sites, and every link is delivered to both threads
+// of a pair.
 // Measured (B200, three prepared states in turn) against warps of 16 consecutive flat sites, whose link loads are two
 // half-used runs, in blocks of 128 threads with separate memsets: S_e^dag S_e of three fields at 6x10x14x18 51.3 ->
-// 43.0 us, D at 24^3x48 201 -> 198 us, D^dag of 12 fields at 16^3x32 unchanged (415 us), D at 8^4 unchanged.  On the
-// same buffers every call: D at 24^3x48 187 -> 174 us, three fields at 6x10x14x18 19.6 -> 16.8 us.
+// 43.0 us, D at 24^3x48 201 -> 198 us, D^dag of 12 fields at 16^3x32 415 -> 379 us (by the grid order: fields
+// fastest), D at 8^4 unchanged; in graphs of calls 8 k sites x fields 5.5 -> 5.8 us, 10^4 sites x 4 17.3 -> 14.9 us.
+// On the same buffers every call: D at 24^3x48 187 -> 174 us, three fields at 6x10x14x18 19.6 -> 16.8 us.
 // Measured and not kept: 4D site tiles per block (187-227 us at 24^3x48), two to four fields per pair on one link
 // load (376-391 against 393 us for the 12 fields, at 8-12 warps per SM), the four directions on four warps (256 us).
 #pragma once
